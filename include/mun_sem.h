@@ -123,8 +123,13 @@ typedef struct {
                                  strip kernel's ticks in one cooperative launch, each CTA
                                  waiting only for its four neighbours' previous tick, for
                                  one-order groups whose chunks are all resident at once;
-                                 otherwise the strip kernel per tick); auto picks strips
-                                 when the batch has at least one strip per SM            */
+                                 otherwise the strip kernel per tick), 5 resident kernels
+                                 (cooperative launches that march a wave of solves through
+                                 all time steps with the wavefield in shared memory).
+                                 auto, with tile, strip_bands and graph_chunk left 0: the
+                                 resident kernels for every solve that fits the SMs (5
+                                 chooses the same way) and, for the rest, strips when the
+                                 batch has at least one strip per SM, else tiles         */
   int32_t strip_bands;        /* strip kernel: element rows per CTA; 0 = automatic
                                  (full-height strips when the batch's strips give 2
                                  CTAs per SM, else chunks of >= 4 rows so that strips
@@ -152,22 +157,23 @@ int sem_run(sem_batch_t* batch, const sem_solve_t* solves, int32_t n,
             const sem_launch_cfg_t* cfg, void* stream);
 /* number of kernel launches issued by the last sem_run (for accounting) */
 int64_t sem_batch_last_launches(const sem_batch_t* batch);
-/* number of consecutive groups the last sem_run ran (1 unless ckpt_k = 0 solves were
- * split under the memory budget) */
+/* number of consecutive groups the last sem_run ran: waves of the resident kernels and
+ * groups of the others (1 unless ckpt_k = 0 solves were split under the memory budget) */
 int32_t sem_batch_last_groups(const sem_batch_t* batch);
-/* launch shape the last sem_run used: tile kernel tile (elements) and strip kernel
- * element rows per CTA (0 when the tile kernel ran); any pointer may be NULL */
+/* launch shape the last sem_run used: tile of the tile or resident kernels (elements) and
+ * strip kernel element rows per CTA (0 otherwise); any pointer may be NULL */
 int sem_batch_last_shape(const sem_batch_t* batch, int32_t* tile_ex, int32_t* tile_ez,
                          int32_t* strip_bands);
 /* tick rounds the last sem_run launched, summed over its groups (each round launches the
- * tick kernel once per polynomial order, then the tick counter kernel) */
+ * tick kernel once per polynomial order, then the tick counter kernel; the resident kernels
+ * count their time steps) */
 int64_t sem_batch_last_ticks(const sem_batch_t* batch);
 /* device time of the last sem_run's tick loops (CUDA events recorded on its stream
  * around each group's tick launches; set-up and output kernels excluded), in ms.
  * Waits for those events. */
 int sem_batch_last_tick_ms(const sem_batch_t* batch, double* ms_out);
 /* kernel variant used by the last sem_run: 1 tile, 2 strip, 3 persistent tile,
- * 4 persistent strip */
+ * 4 persistent strip, 5 resident */
 int32_t sem_batch_last_kernel(const sem_batch_t* batch);
 
 /* Single-solve conveniences (plain path): forward with receivers in the run()

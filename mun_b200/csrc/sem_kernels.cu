@@ -144,6 +144,14 @@ struct SolveDev {
   // for t = 0 .. nt (row t), written by forward and replay ticks
   const float* bnd_coef;
   float* bnd_hist;
+  // resident kernels: per tile the quads (row << 16 | element: one row of an element's own nodes)
+  // that receivers reach, per quad its terms in receiver order (receiver of the tile << 8 | mask of
+  // the nodes) and their weights
+  const int* iq_off;
+  const int* iq_pos;
+  const int* iterm_off;
+  const int* iterm;
+  const float* iterm_w;
 };
 
 __device__ __forceinline__ void decode(const SolveDev& s, int sig, int& act, int& t, int& seg) {
@@ -1904,6 +1912,8 @@ __global__ void __launch_bounds__(kStripCols, (N <= 4) ? SEM_STRIP_MIN_BLOCKS : 
   }
 }
 
+#include "sem_resident.cuh"
+
 // Diagnostics of the device waits' time limits, without any fault: which = 0 waits on an
 // mbarrier whose expected bytes never arrive (no copy is issued), 1 on a grid barrier one
 // arrival short of its target (cooperative launch of 2 CTAs), 2 on a grid barrier that
@@ -2065,10 +2075,22 @@ struct sem_plan_s {
   float* rec_w = nullptr;
   int* node_pos = nullptr;
   std::vector<int> h_rec_base;
+  std::vector<float> h_rec_w;
   // receiver lists per tile (tile kernel, key (tile_ex, tile_ez)) or per strip band
   // (strip kernel, key (-1, elements per strip)): device arrays rec_off/ids, inj_off/ids
   struct Lists { int* rec_off; int* rec_ids; int* inj_off; int* inj_ids; };
   mutable std::map<std::pair<int, int>, Lists> lists;
+  // resident kernels: lists of a balanced tiling, key (tiles in x, tiles in z), with the largest
+  // counts of any tile (read-out receivers, injection receivers, quads and terms)
+  struct ResLists {
+    Lists l;
+    int *iq_off, *iq_pos, *iterm_off, *iterm;
+    float* iterm_w;
+    int nrec, ninj, nquad, nterm;
+  };
+  mutable std::map<std::pair<int, int>, ResLists> res_lists;
+  // their tilings by (adjoint, most elements per tile)
+  mutable std::map<std::pair<bool, int>, std::pair<int, int>> res_tilings;
   mutable std::mutex mu;
 };
 
@@ -2362,12 +2384,13 @@ TensorMapEncodeTiledFn tensor_map_encoder() {
   });
   return fn;
 }
-int encode_band_map(CUtensorMap* m, char* ws_base, const sem_plan_s* p, long long nslots) {
+// (bw, bh): the box, by default the strip kernel's band
+int encode_band_map(CUtensorMap* m, char* ws_base, const sem_plan_s* p, long long nslots, int bw = 0, int bh = 0) {
   TensorMapEncodeTiledFn enc = tensor_map_encoder();
   if (!enc) return fail(SEM_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
   const cuuint64_t dims[3] = {(cuuint64_t)p->pitch, (cuuint64_t)p->nzg, (cuuint64_t)nslots};
   const cuuint64_t strides[2] = {(cuuint64_t)p->pitch * 4, (cuuint64_t)p->fstride * 4};
-  const cuuint32_t box[3] = {(cuuint32_t)strip_bw(p->npol), (cuuint32_t)(p->npol + 1), 1};
+  const cuuint32_t box[3] = {(cuuint32_t)(bw ? bw : strip_bw(p->npol)), (cuuint32_t)(bh ? bh : p->npol + 1), 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, ws_base, dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -2436,6 +2459,9 @@ struct sem_batch_s {
   CUtensorMap* d_tmaps = nullptr;       // strip kernel: band-load tensor map of each solve
   int tmaps_cap = 0;
   std::vector<CUtensorMap> h_tmaps;
+  unsigned long long* d_ll = nullptr;   // resident kernels: exchange words, and the last step tag
+  long long ll_cap = 0;                 //   used (tags only grow, so stale words never match)
+  unsigned ll_tag = 0;
   char* d_sync = nullptr;               // persistent strip kernel: per-CTA tick counters and
   long long sync_cap = 0;               //   per-solve barrier counters
 };
@@ -2472,6 +2498,8 @@ int sem_plan_create(const sem_plan_desc_t* d, sem_plan_t** out) {
     pos[i] = (int)((g / nxg) * p->pitch + (g % nxg));
   }
   p->h_rec_base.assign(d->rec_base, d->rec_base + 2 * d->nrec);
+  p->h_rec_w.resize((size_t)d->nrec * NP * NP);
+  for (size_t i = 0; i < p->h_rec_w.size(); ++i) p->h_rec_w[i] = (float)d->rec_w[i];
   for (int r = 0; r < d->nrec; ++r) {
     const int bx = p->h_rec_base[2 * r], bz = p->h_rec_base[2 * r + 1];
     if (bx < 0 || bz < 0 || bx % d->npol || bz % d->npol || bx + d->npol > nxg - 1 ||
@@ -2542,6 +2570,12 @@ int sem_plan_destroy(sem_plan_t* p) {
     cudaFree(kv.second.rec_off); cudaFree(kv.second.rec_ids);
     cudaFree(kv.second.inj_off); cudaFree(kv.second.inj_ids);
   }
+  for (auto& kv : p->res_lists) {
+    cudaFree(kv.second.l.rec_off); cudaFree(kv.second.l.rec_ids);
+    cudaFree(kv.second.l.inj_off); cudaFree(kv.second.l.inj_ids);
+    cudaFree(kv.second.iq_off); cudaFree(kv.second.iq_pos);
+    cudaFree(kv.second.iterm_off); cudaFree(kv.second.iterm); cudaFree(kv.second.iterm_w);
+  }
   delete p;
   return SEM_OK;
 }
@@ -2568,7 +2602,7 @@ int sem_batch_destroy(sem_batch_t* b) {
   for (cudaEvent_t e : b->tick_ev) cudaEventDestroy(e);
   cudaFree(b->d_io);
   cudaFree(b->arena); cudaFree(b->d_tick); cudaFree(b->d_solves); cudaFree(b->d_cta); cudaFree(b->d_tmaps);
-  cudaFree(b->d_sync);
+  cudaFree(b->d_sync); cudaFree(b->d_ll);
   delete b;
   return SEM_OK;
 }
@@ -2578,6 +2612,18 @@ int64_t sem_batch_last_launches(const sem_batch_t* b) { return b ? b->last_launc
 int32_t sem_batch_last_kernel(const sem_batch_t* b) { return b ? b->last_kernel : -1; }
 
 }  // extern "C"
+
+// what every solve of a batch must bring
+static int check_solve(const sem_batch_t* b, const sem_solve_t& s) {
+  if (!s.plan || !s.velocity || !s.rec_out) return fail(SEM_ERR_ARG, "solve missing plan/velocity/rec_out");
+  const bool adj = s.flags & SEM_F_ADJOINT;
+  if (adj && !(s.flags & SEM_F_SHIFT)) return fail(SEM_ERR_ARG, "adjoint requires the shifted receiver convention");
+  if ((adj || (s.flags & SEM_F_MISFIT)) && !s.y_obs) return fail(SEM_ERR_ARG, "y_obs required");
+  if (s.decim < 1 || s.it0 < 0 || s.it1 > s.plan->nt || s.it0 >= s.it1)
+    return fail(SEM_ERR_ARG, "bad misfit window");
+  if (s.plan->device != b->device) return fail(SEM_ERR_ARG, "plan and batch on different devices");
+  return SEM_OK;
+}
 
 // One group of solves run to completion: the whole batch, or one group of an automatic
 // schedule (solves then carry the group's checkpoint interval).
@@ -2591,12 +2637,7 @@ static int run_group(sem_batch_t* b, const sem_solve_t* solves, int32_t n,
   long long total = 0;
   for (int i = 0; i < n; ++i) {
     const sem_solve_t& s = solves[i];
-    if (!s.plan || !s.velocity || !s.rec_out) return fail(SEM_ERR_ARG, "solve missing plan/velocity/rec_out");
     const bool adj = s.flags & SEM_F_ADJOINT;
-    if (adj && !(s.flags & SEM_F_SHIFT)) return fail(SEM_ERR_ARG, "adjoint requires the shifted receiver convention");
-    if ((adj || (s.flags & SEM_F_MISFIT)) && !s.y_obs) return fail(SEM_ERR_ARG, "y_obs required");
-    if (s.decim < 1 || s.it0 < 0 || s.it1 > s.plan->nt || s.it0 >= s.it1)
-      return fail(SEM_ERR_ARG, "bad misfit window");
     kk[i] = adj ? std::max(2, std::min((int)s.ckpt_k, s.plan->nt)) : 2;
     ws[i] = layout(s.plan, s.flags, kk[i], &nseg[i]);
     total += ws[i].bytes;
@@ -2654,7 +2695,6 @@ static int run_group(sem_batch_t* b, const sem_solve_t* solves, int32_t n,
     const int i = order[oi];
     const sem_solve_t& s = solves[i];
     const sem_plan_s* p = s.plan;
-    if (p->device != b->device) return fail(SEM_ERR_ARG, "plan and batch on different devices");
     sem_plan_s::Lists L;
     int ntx, ntz, ntiles, rc;
     if (use_strip) {
@@ -3090,6 +3130,8 @@ int auto_schedule(const sem_solve_t* sv, int n, const sem_launch_cfg_t& cfg, lon
 
 }  // namespace
 
+#include "sem_resident_run.cuh"
+
 extern "C" {
 
 int sem_run(sem_batch_t* b, const sem_solve_t* solves, int32_t n, const sem_launch_cfg_t* cfg_in,
@@ -3100,9 +3142,9 @@ int sem_run(sem_batch_t* b, const sem_solve_t* solves, int32_t n, const sem_laun
   sem_launch_cfg_t cfg = cfg_in ? *cfg_in : sem_launch_cfg_t{0, 0, 256, 0, 0, 0, 0};
   if (!(cfg.tile_ex == 0 && cfg.tile_ez == 0) && (cfg.tile_ex < 1 || cfg.tile_ez < 1))
     return fail(SEM_ERR_ARG, "tile size must be >= 1 (or 0 x 0: automatic)");
-  if (cfg.kernel < 0 || cfg.kernel > 4)
+  if (cfg.kernel < 0 || cfg.kernel > 5)
     return fail(SEM_ERR_ARG,
-                "kernel must be 0 (auto), 1 (tile), 2 (strip), 3 (persistent tile), 4 (persistent strip)");
+                "kernel must be 0 (auto), 1 (tile), 2 (strip), 3 (persistent tile), 4 (persistent strip), 5 (resident)");
   if (cfg.threads < 32 || cfg.threads > 256 || cfg.threads % 32) cfg.threads = 256;
   if (cfg.memory_budget < 0) return fail(SEM_ERR_ARG, "memory_budget must be >= 0");
   if (cfg.strip_bands < 0) return fail(SEM_ERR_ARG, "strip_bands must be >= 0");
@@ -3113,8 +3155,28 @@ int sem_run(sem_batch_t* b, const sem_solve_t* solves, int32_t n, const sem_laun
   if (n == 0) return SEM_OK;
   bool any_auto = false;
   for (int i = 0; i < n; ++i) {
-    if (!solves[i].plan) return fail(SEM_ERR_ARG, "solve missing plan/velocity/rec_out");
+    if (int rc = check_solve(b, solves[i])) return rc;
     any_auto |= (solves[i].flags & SEM_F_ADJOINT) && solves[i].ckpt_k <= 0;
+  }
+  long long budget = cfg.memory_budget;
+  const bool resident = cfg.kernel == 5 || (cfg.kernel == 0 && cfg.graph_chunk <= 0 && cfg.tile_ex == 0 && cfg.strip_bands == 0);
+  if (budget == 0 && (any_auto || resident)) {
+    size_t fr = 0, tot = 0;
+    CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+    budget = (long long)(0.85 * (double)((long long)fr + b->arena_bytes)) - (512LL << 20);
+    budget = std::max(budget, 1LL << 20);
+  }
+  std::vector<sem_solve_t> left;
+  if (resident) {
+    std::vector<int> rest;
+    if (int rc = run_resident(b, solves, n, budget, stream, &rest)) return rc;
+    if (rest.empty()) return SEM_OK;
+    if (cfg.kernel == 5) cfg.kernel = 0;
+    for (int i : rest) left.push_back(solves[i]);
+    solves = left.data();
+    n = (int32_t)left.size();
+    any_auto = false;
+    for (int i = 0; i < n; ++i) any_auto |= (solves[i].flags & SEM_F_ADJOINT) && solves[i].ckpt_k <= 0;
   }
   if (cfg.tile_ex == 0) {
     int dev = 0, sms = 148;
@@ -3125,15 +3187,8 @@ int sem_run(sem_batch_t* b, const sem_solve_t* solves, int32_t n, const sem_laun
   b->last_tile_ex = cfg.tile_ex;
   b->last_tile_ez = cfg.tile_ez;
   if (!any_auto) {
-    b->last_groups = 1;
+    b->last_groups++;
     return run_group(b, solves, n, cfg, stream);
-  }
-  long long budget = cfg.memory_budget;
-  if (budget == 0) {
-    size_t fr = 0, tot = 0;
-    CUDA_TRY(cudaMemGetInfo(&fr, &tot));
-    budget = (long long)(0.85 * (double)((long long)fr + b->arena_bytes)) - (512LL << 20);
-    budget = std::max(budget, 1LL << 20);
   }
   std::vector<GroupPlan> groups;
   int rc = auto_schedule(solves, n, cfg, budget, &groups);
