@@ -2089,8 +2089,9 @@ struct sem_plan_s {
     int nrec, ninj, nquad, nterm;
   };
   mutable std::map<std::pair<int, int>, ResLists> res_lists;
-  // their tilings by (adjoint, most elements per tile)
-  mutable std::map<std::pair<bool, int>, std::pair<int, int>> res_tilings;
+  struct ResCounts { int nrec = 0, ninj = 0, nquad = 0, nterm = 0; };  // bounds over a tiling's tiles
+  struct ResTiling { int tx = 0, tz = 0; ResCounts n; };
+  mutable std::map<std::tuple<int, bool, int>, ResTiling> res_tilings;  // by lanes per element, adjoint, capacity
   mutable std::mutex mu;
 };
 

@@ -21,10 +21,9 @@
 // later, after words that its readers sent when they were done with it (two steps
 // suffice for direct neighbours, three for the corner node).
 //
-// Threads.  A compute thread owns a column of elements: lane by lane the elements of a tile row,
-// stepping down the element rows of its chunk.  All lines of an element are evaluated in its
-// registers (480 independent fused multiply-adds at N = 4: the fp32 pipe, not latency, is the
-// limit); the carry into the element below stays in registers, the carry into the right
+// Threads.  A compute thread owns a column of elements, or of their halves: lane by lane the
+// elements of a tile row, stepping down the element rows of its chunk.  All lines of an element
+// are evaluated in registers; the carry into the element below stays in registers, the carry into the right
 // neighbour goes by shuffle, and the first lane of a row is the left halo element, evaluated
 // for its carry only.  A chunk starts with the z-lines of the element row above it, for their
 // carry.  Nodes are advanced into the other of two buffers and each warp sends its own edge
@@ -34,9 +33,9 @@
 // Arithmetic.  Per node the operations and roundings of the tile and strip kernels, in the
 // same order: results are bitwise equal to theirs.
 
-// most threads of a resident CTA: 168 registers each forward, 255 adjoint (with 128 / 168 they
-// spill, and a step of 128 models takes 47 / 113 us instead of 46 / 105)
-__host__ __device__ constexpr int res_threads(bool adj) { return adj ? 256 : 384; }
+// most threads of a resident CTA, by lanes per element: 168 (forward) and 255 (adjoint) registers
+// each with one, 128 with two
+__host__ __device__ constexpr int res_threads(int lpe, bool adj) { return lpe == 2 ? 512 : adj ? 256 : 384; }
 constexpr int kResSlots = 4;       // exchange slots by step tag
 
 // Shared-memory layout (float offsets) and exchange layout (words) of one launch, by its
@@ -129,17 +128,17 @@ __host__ __device__ inline bool res_range(int kind, int idx, int nt, int k, int 
   return true;
 }
 
-// The z-lines of one element, two columns at a time as the halves of packed FFMA2 / FMUL2 (per
+// The z-lines of NQ pairs of an element's columns, a pair at a time as the halves of packed FFMA2 / FMUL2 (per
 // half the scalar sequence), from its rows of nodes u (field), c (c^2) and, adjoint, w (forward
 // field): segment results of row i in Z[i], sensitivities in S[i]; with CARRY only the last
 // row's, for the element below.
-template <int N, bool ADJ, bool CARRY>
-__device__ __forceinline__ void res_zlines(const float2 (&u)[N + 1][(N + 1) / 2], const float2 (&c)[N + 1][(N + 1) / 2],
-                                           const float2 (&w)[N + 1][(N + 1) / 2], float2 (&Z)[N + 1][(N + 1) / 2],
-                                           float2 (&S)[N + 1][(N + 1) / 2]) {
-  constexpr int NP = N + 1, H2 = (N + 1) / 2;
+template <int N, int NQ, bool ADJ, bool CARRY>
+__device__ __forceinline__ void res_zlines(const float2 (&u)[N + 1][NQ], const float2 (&c)[N + 1][NQ],
+                                           const float2 (&w)[N + 1][NQ], float2 (&Z)[N + 1][NQ],
+                                           float2 (&S)[N + 1][NQ]) {
+  constexpr int NP = N + 1;
 #pragma unroll
-  for (int p = 0; p < H2; ++p) {
+  for (int p = 0; p < NQ; ++p) {
     // (the independent sums side by side, so that consecutive instructions do not wait)
     float2 d[NP], q[NP];
 #pragma unroll
@@ -216,13 +215,16 @@ __device__ __forceinline__ void res_xline(const float (&u)[N + 1], const float (
 // nc: compute threads (the first of the CTA); the rest serve the receivers.  sw: lanes per tile
 // row (a power of two, at least the tile's columns of elements + 2: one for the left halo, one
 // for the nodes on the right); ezc: element rows per chunk.
-template <int N, bool ADJ, bool STC>
-__global__ void __launch_bounds__(res_threads(ADJ), 1)
+template <int N, int LPE, bool ADJ, bool STC>
+__global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
     sem_resident_kernel(const SolveDev* __restrict__ solves, const int* __restrict__ cta_solve,
                         const __grid_constant__ ResLay L, unsigned long long* __restrict__ ll,
                         const unsigned tag0, const int kind, const int idx, const int nc, const int sw,
                         const int ezc) {
   constexpr int NP = N + 1, H2 = (N + 1) / 2;
+  // two lanes per element (order 4): each has two columns' z-lines and two rows' x-lines and nodes
+  static_assert(LPE == 1 || N == 4, "an element's halves");
+  constexpr int NJ = N / LPE, NQ = LPE == 2 ? 1 : H2;
   extern __shared__ __align__(128) float sm[];
   __shared__ SolveDev S;
   __shared__ int s_fail;
@@ -324,7 +326,7 @@ __global__ void __launch_bounds__(res_threads(ADJ), 1)
         else if ((q -= n_b) < n_l) { r = q; cc = 0; to = (blk - 1) * llc + L.ll_r + q; }
         else if ((q -= n_l) < n_t) { r = 0; cc = q; to = (blk - S.tiles_x) * llc + L.ll_b + q; }
         else { r = 0; cc = 0; to = (blk - S.tiles_x - 1) * llc + L.ll_c; }
-        const int wp = (((r / N) / ezc) * sw + cc / N + 1) >> 5;
+        const int wp = (((r / N) / ezc) * sw + (cc / N + 1) * LPE + (r % N) / NJ) >> 5;
         const int at = atomicAdd(&s_wo[pass ? wp : wp + 1], 1);
         if (pass) wout[at] = make_int2(o0 + r * L.Wp + cc, to);
       }
@@ -507,14 +509,14 @@ __global__ void __launch_bounds__(res_threads(ADJ), 1)
   float rs_next = 0.f;
   if (ADJ && my_rec && nst > 2) rs_next = residual(t_hi - 3);
 
-  // ---------------- compute threads: element column sl - 1 of the tile (lane 0 of a row: the
-  // left halo; after the last element: the lane of the nodes on its right, the mesh's last column
-  // or the right neighbour's first)
-  const int sl = tid & (sw - 1), ch = tid / sw;
-  const int ec = min(sl - 1, Q.EX);             // lanes past that repeat it
-  const bool full = sl >= 1 && sl <= Q.EX;
-  const bool owner = full || (sl == Q.EX + 1 && !Q.hr);
-  const bool no_left = sl == 1 && !Q.hl;
+  // ---------------- compute threads: element column ec of the tile (the first of a row: the left
+  // halo; after the last element: the nodes on its right, the mesh's last column or the right
+  // neighbour's first)
+  const int el = (tid & (sw - 1)) / LPE, h = tid % LPE, ch = tid / sw;
+  const int ec = min(el - 1, Q.EX);             // lanes past that repeat it
+  const bool full = el >= 1 && el <= Q.EX;
+  const bool owner = full || (el == Q.EX + 1 && !Q.hr);
+  const bool no_left = el == 1 && !Q.hl;
   const int EZ1 = Q.EZ + (Q.hb ? 0 : 1);        // rows of elements; the mesh's last line is one more
   const int er_lo = ch * ezc, er_hi = min(EZ1, er_lo + ezc);
   const bool damp = !STC && (!ADJ || (S.flags & F_EXACT));
@@ -609,53 +611,70 @@ __global__ void __launch_bounds__(res_threads(ADJ), 1)
 
     // ---- down the chunk's element rows; the carry of the row above comes first.  The rows of
     // nodes stay in registers: an element's last row is the next one's first
-    float2 u[NP][H2], c[NP][H2], w[NP][H2];
+    float2 u[NP][NQ], c[NP][NQ], w[NP][NQ];
     auto load = [&](const int a, const int o) {
-      get2<N>(fb + o, u[a]);
-      get2<N>(sm + L.c + o, c[a]);
-      if (ADJ) get2<N>(fw + o, w[a]);
+      if constexpr (LPE == 2) {
+        u[a][0] = *reinterpret_cast<const float2*>(fb + o);
+        c[a][0] = *reinterpret_cast<const float2*>(sm + L.c + o);
+        if (ADJ) w[a][0] = *reinterpret_cast<const float2*>(fw + o);
+      } else {
+        get2<N>(fb + o, u[a]);
+        get2<N>(sm + L.c + o, c[a]);
+        if (ADJ) get2<N>(fw + o, w[a]);
+      }
     };
-    float2 zc[H2], szc[H2];
+    const int oz = oc + (LPE == 2 ? 2 * h : 0);
+    float2 zc[NQ], szc[NQ];
 #pragma unroll
-    for (int i = 0; i < H2; ++i) { zc[i] = make_float2(0.f, 0.f); szc[i] = make_float2(0.f, 0.f); }
+    for (int i = 0; i < NQ; ++i) { zc[i] = make_float2(0.f, 0.f); szc[i] = make_float2(0.f, 0.f); }
     {
-      const int o = oc + min(er_lo, EZ1 - 1) * N * L.Wp;
+      const int o = oz + min(er_lo, EZ1 - 1) * N * L.Wp;
       load(N, o);
       if (er_lo < er_hi && (er_lo > 0 || Q.ht)) {
-        float2 Z[NP][H2], SZ[NP][H2];
+        float2 Z[NP][NQ], SZ[NP][NQ];
 #pragma unroll
         for (int a = 0; a < N; ++a) load(a, o + (a - N) * L.Wp);
-        res_zlines<N, ADJ, true>(u, c, w, Z, SZ);
+        res_zlines<N, NQ, ADJ, true>(u, c, w, Z, SZ);
 #pragma unroll
-        for (int i = 0; i < H2; ++i) { zc[i] = Z[N][i]; if (ADJ) szc[i] = SZ[N][i]; }
+        for (int i = 0; i < NQ; ++i) { zc[i] = Z[N][i]; if (ADJ) szc[i] = SZ[N][i]; }
       }
     }
-    // the next element's first node of a row is the next lane's
-    auto beyond = [&](const float2 (&f)[H2]) { return __shfl_down_sync(0xffffffffu, f[0].x, 1, sw); };
+    // the next element's first node of a row is the next element's lane's
+    auto beyond = [&](const float2 (&f)[H2]) { return __shfl_down_sync(0xffffffffu, f[0].x, LPE, sw); };
 #pragma unroll 1
     for (int k = 0; k < ezc; ++k) {
       const int er = er_lo + k;
       // rows of lanes whose chunk has ended keep the warp's shuffles company
       const bool on = er < er_hi;
       if (!__any_sync(0xffffffffu, on)) break;
-      const int e_ = min(er, EZ1 - 1), r0 = e_ * N;
+      const int e_ = min(er, EZ1 - 1), r0 = e_ * N + h * NJ;
       const bool vz = e_ == Q.EZ;  // the mesh's last line of nodes: one row, no lines below
-      const int o = oc + e_ * N * L.Wp;
 #pragma unroll
-      for (int i = 0; i < H2; ++i) { u[0][i] = u[N][i]; c[0][i] = c[N][i]; if (ADJ) w[0][i] = w[N][i]; }
+      for (int i = 0; i < NQ; ++i) { u[0][i] = u[N][i]; c[0][i] = c[N][i]; if (ADJ) w[0][i] = w[N][i]; }
 #pragma unroll
-      for (int a = 1; a < NP; ++a) load(a, o + a * L.Wp);
-      float ux[N], cx[N], wx[N];
+      for (int a = 1; a < NP; ++a) load(a, oz + (e_ * N + a) * L.Wp);
+      // this lane's rows: N nodes each and the one beyond
+      float2 xu[NJ][H2], xc[NJ][H2], xw[NJ][H2];
+      float ux[NJ], cx[NJ], wx[NJ];
 #pragma unroll
-      for (int a = 0; a < N; ++a) {
-        ux[a] = beyond(u[a]);
-        cx[a] = beyond(c[a]);
-        wx[a] = ADJ ? beyond(w[a]) : 0.f;
+      for (int j = 0; j < NJ; ++j) {
+        if constexpr (LPE == 2) {
+          const int o = oc + (r0 + j) * L.Wp;
+          get2<N>(fb + o, xu[j]);
+          get2<N>(sm + L.c + o, xc[j]);
+          if (ADJ) get2<N>(fw + o, xw[j]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < H2; ++i) { xu[j][i] = u[j][i]; xc[j][i] = c[j][i]; if (ADJ) xw[j][i] = w[j][i]; }
+        }
+        ux[j] = beyond(xu[j]);
+        cx[j] = beyond(xc[j]);
+        wx[j] = ADJ ? beyond(xw[j]) : 0.f;
       }
-      float2 Z[NP][H2], SZ[NP][H2];
-      res_zlines<N, ADJ, false>(u, c, w, Z, SZ);
+      float2 Z[NP][NQ], SZ[NP][NQ];
+      res_zlines<N, NQ, ADJ, false>(u, c, w, Z, SZ);
 #pragma unroll
-      for (int i = 0; i < H2; ++i) {
+      for (int i = 0; i < NQ; ++i) {
         Z[0][i] = vz ? zc[i] : __fadd2_rn(zc[i], Z[0][i]);
         zc[i] = Z[N][i];
         if (ADJ) {
@@ -664,76 +683,94 @@ __global__ void __launch_bounds__(res_threads(ADJ), 1)
           szc[i] = SZ[N][i];
         }
       }
+      // the z results of this lane's rows: two lanes per element swap the halves they have for each other
+      float2 Zr[NJ][H2], SZr[NJ][H2];
+      auto rows_of = [&](const float2 (&F)[NP][NQ], float2 (&R)[NJ][H2]) {
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          if constexpr (LPE == 2) {
+            const float2 give = h ? F[j][0] : F[NJ + j][0], own = h ? F[NJ + j][0] : F[j][0];
+            const float2 got = make_float2(__shfl_xor_sync(0xffffffffu, give.x, 1), __shfl_xor_sync(0xffffffffu, give.y, 1));
+            R[j][0] = h ? got : own;
+            R[j][H2 - 1] = h ? own : got;
+          } else {
+#pragma unroll
+            for (int i = 0; i < H2; ++i) R[j][i] = F[j][i < NQ ? i : 0];
+          }
+        }
+      };
+      rows_of(Z, Zr);
+      if (ADJ) rows_of(SZ, SZr);
 
       // ---- the element's rows of owned nodes: x-lines, then the update
       const int ri = oc + r0 * L.Wp, oi = r0 * L.Cp + ec * N;
-      float2 X[N][H2], SX[N][H2];
-      float re[N], rs[N];
+      float2 X[NJ][H2], SX[NJ][H2];
+      float re[NJ], rs[NJ];
 #pragma unroll
-      for (int j = 0; j < N; ++j) {
+      for (int j = 0; j < NJ; ++j) {
         float lu[NP], lc[NP], lw[NP];
 #pragma unroll
-        for (int i = 0; i < N; ++i) { lu[i] = lane_of(u[j], i); lc[i] = lane_of(c[j], i); if (ADJ) lw[i] = lane_of(w[j], i); }
+        for (int i = 0; i < N; ++i) { lu[i] = lane_of(xu[j], i); lc[i] = lane_of(xc[j], i); if (ADJ) lw[i] = lane_of(xw[j], i); }
         lu[N] = ux[j]; lc[N] = cx[j]; if (ADJ) lw[N] = wx[j];
         res_xline<N, ADJ>(lu, lc, lw, X[j], SX[j], re[j], rs[j]);
       }
 #pragma unroll
-      for (int j = 0; j < N; ++j) {
-        re[j] = __shfl_up_sync(0xffffffffu, re[j], 1, sw);
+      for (int j = 0; j < NJ; ++j) {
+        re[j] = __shfl_up_sync(0xffffffffu, re[j], LPE, sw);
         if (no_left) re[j] = 0.f;
         X[j][0].x = full ? __fadd_rn(re[j], X[j][0].x) : re[j];
         if (ADJ) {
-          rs[j] = __shfl_up_sync(0xffffffffu, rs[j], 1, sw);
+          rs[j] = __shfl_up_sync(0xffffffffu, rs[j], LPE, sw);
           if (no_left) rs[j] = 0.f;
           SX[j][0].x = full ? __fadd_rn(rs[j], SX[j][0].x) : rs[j];
         }
       }
       // (nodes past the mesh's last line or column lie in this tile's arrays too and stay 0)
       const bool mine = owner && on;
-      float4 tz[N];   // 1/m_z and R_z, twice each
-      float2 ndz[N];
+      float4 tz[NJ];   // 1/m_z and R_z, twice each
+      float2 ndz[NJ];
 #pragma unroll
-      for (int j = 0; j < N; ++j) {
+      for (int j = 0; j < NJ; ++j) {
         tz[j] = *reinterpret_cast<const float4*>(sm + L.tz + 8 * (r0 + j));
         ndz[j] = *reinterpret_cast<const float2*>(sm + L.tz + 8 * (r0 + j) + 4);
       }
       if constexpr (ADJ) {
-        float2 g[N][H2];
+        float2 g[NJ][H2];
 #pragma unroll
-        for (int j = 0; j < N; ++j) get2<N>(sm + L.g + oi + j * L.Cp, g[j]);
+        for (int j = 0; j < NJ; ++j) get2<N>(sm + L.g + oi + j * L.Cp, g[j]);
 #pragma unroll
-        for (int j = 0; j < N; ++j)
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
           for (int i = 0; i < H2; ++i)
-            SX[j][i] = __ffma2_rn(make_float2(tz[j].z, tz[j].w), SX[j][i], __fmul2_rn(Rx[i], SZ[j][i]));  // sens_increment
+            SX[j][i] = __ffma2_rn(make_float2(tz[j].z, tz[j].w), SX[j][i], __fmul2_rn(Rx[i], SZr[j][i]));  // sens_increment
         if (stc_edge && t <= S.nt - 2 && mine) {
           // g lambda (b_{t+2} - b_t) at the absorbing edges, rounded as bnd_sens
 #pragma unroll
-          for (int j = 0; j < N; ++j)
+          for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int i = 0; i < N; ++i) {
               const int k = edge_of(r0 + j, ec * N + i);
               if (k >= 0) {
                 float& f = (i & 1) ? SX[j][i / 2].y : SX[j][i / 2].x;
-                f = __fadd_rn(f, __fmul_rn(__fmul_rn(sm[L.be + 2 * bn + k], lane_of(u[j], i)), sm[L.bd + (t & 1) * bn + k]));
+                f = __fadd_rn(f, __fmul_rn(__fmul_rn(sm[L.be + 2 * bn + k], lane_of(xu[j], i)), sm[L.bd + (t & 1) * bn + k]));
               }
             }
         }
 #pragma unroll
-        for (int j = 0; j < N; ++j)
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
           for (int i = 0; i < H2; ++i) g[j][i] = __fadd2_rn(g_start ? make_float2(0.f, 0.f) : g[j][i], SX[j][i]);
         if (mine) {
 #pragma unroll
-          for (int j = 0; j < N; ++j) put2<N>(sm + L.g + oi + j * L.Cp, g[j]);
+          for (int j = 0; j < NJ; ++j) put2<N>(sm + L.g + oi + j * L.Cp, g[j]);
         }
       }
-      float2 v[N][H2];
+      float2 v[NJ][H2];
 #pragma unroll
-      for (int j = 0; j < N; ++j) get2<N>(sm + L.v + oi + j * L.Cp, v[j]);
+      for (int j = 0; j < NJ; ++j) get2<N>(sm + L.v + oi + j * L.Cp, v[j]);
       if constexpr (STC) {
 #pragma unroll
-        for (int j = 0; j < N; ++j) {
+        for (int j = 0; j < NJ; ++j) {
           const int r = r0 + j;
           const bool top = Q.gz0 + r == 0;
           int m = 0;
@@ -750,7 +787,7 @@ __global__ void __launch_bounds__(res_threads(ADJ), 1)
             if (!ADJ) { if (r == src_r && ec == src_e && i == src_i) ex = s_src[t & 1]; }
             else if (m) ex = sm[L.ia + (t & 1) * (L.niq * N) + (m - 1) * N + i];
             float rr, vv;
-            advance_node_stacey(ADJ, lane_of(u[j], i), lane_of(v[j], i), lane_of(X[j], i), lane_of(Z[j], i), -lane_of(nix, i),
+            advance_node_stacey(ADJ, lane_of(xu[j], i), lane_of(v[j], i), lane_of(X[j], i), lane_of(Zr[j], i), -lane_of(nix, i),
                                 lane_of(Rx, i), tz[j].x, tz[j].z, ex, e1, e2, rr, vv);
             if (top) { rr = 0.f; vv = 0.f; }
             if (i & 1) { X[j][i / 2].y = rr; v[j][i / 2].y = vv; } else { X[j][i / 2].x = rr; v[j][i / 2].x = vv; }
@@ -761,13 +798,13 @@ __global__ void __launch_bounds__(res_threads(ADJ), 1)
       } else {
         // as advance_node, two nodes at a time: w = v - P K (the products' signs are exact)
 #pragma unroll
-        for (int j = 0; j < N; ++j)
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
           for (int i = 0; i < H2; ++i)
-            X[j][i] = __ffma2_rn(make_float2(tz[j].z, tz[j].w), X[j][i], __fmul2_rn(Rx[i], Z[j][i]));
+            X[j][i] = __ffma2_rn(make_float2(tz[j].z, tz[j].w), X[j][i], __fmul2_rn(Rx[i], Zr[j][i]));
         if (ADJ && niq > 0 && mine) {
 #pragma unroll
-          for (int j = 0; j < N; ++j) {
+          for (int j = 0; j < NJ; ++j) {
             const int m = imap[(r0 + j) * L.qx + ec];
             if (m) {  // P (injection - K) + mu
               const float* ex = sm + L.ia + (t & 1) * (L.niq * N) + (m - 1) * N;
@@ -780,14 +817,14 @@ __global__ void __launch_bounds__(res_threads(ADJ), 1)
           }
         }
 #pragma unroll
-        for (int j = 0; j < N; ++j)
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
           for (int i = 0; i < H2; ++i)
             v[j][i] = __ffma2_rn(__fmul2_rn(nix[i], make_float2(tz[j].x, tz[j].y)), X[j][i], v[j][i]);
-        if (!ADJ && src_r >= r0 && src_r < r0 + N && ec == src_e) {
+        if (!ADJ && src_r >= r0 && src_r < r0 + NJ && ec == src_e) {
           const float s = s_src[t & 1];
 #pragma unroll
-          for (int j = 0; j < N; ++j)
+          for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int i = 0; i < N; ++i)
               if (i == src_i && r0 + j == src_r) {
@@ -796,16 +833,16 @@ __global__ void __launch_bounds__(res_threads(ADJ), 1)
         }
         bool dq = dxany;
 #pragma unroll
-        for (int j = 0; j < N; ++j) dq |= ndz[j].x != 0.f;
+        for (int j = 0; j < NJ; ++j) dq |= ndz[j].x != 0.f;
 #pragma unroll
-        for (int j = 0; j < N; ++j)
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
-          for (int i = 0; i < H2; ++i) X[j][i] = __fadd2_rn(u[j][i], v[j][i]);
+          for (int i = 0; i < H2; ++i) X[j][i] = __fadd2_rn(xu[j][i], v[j][i]);
         if (damp && dq) {
           // the sponge; elements outside it skip its operations (delta = 0 leaves w and s unchanged);
           // all signs turned: -delta = (-dx)(-dz) + ((-dx) + (-dz))
 #pragma unroll
-          for (int j = 0; j < N; ++j)
+          for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int i = 0; i < H2; ++i) {
               const float2 nl = __ffma2_rn(ndx[i], ndz[j], __fadd2_rn(ndx[i], ndz[j]));
@@ -816,15 +853,15 @@ __global__ void __launch_bounds__(res_threads(ADJ), 1)
       }
       if (mine) {
 #pragma unroll
-        for (int j = 0; j < N; ++j) {
+        for (int j = 0; j < NJ; ++j) {
           put2<N>(fn + ri + j * L.Wp, X[j]);
           put2<N>(sm + L.v + oi + j * L.Cp, v[j]);
         }
         if (!ADJ && bo) {
           float* const p = bo + (Q.gz0 + r0) * pitch + Q.gx0 + ec * N;
 #pragma unroll
-          for (int j = 0; j < N; ++j)
-            if (j == 0 || !vz) {
+          for (int j = 0; j < NJ; ++j)
+            if ((j == 0 && h == 0) || !vz) {
               if constexpr (N == 4) {  // (the row's padding takes the rest of the last node's quad)
                 *reinterpret_cast<float4*>(p + j * pitch) = make_float4(X[j][0].x, X[j][0].y, X[j][H2 - 1].x, X[j][H2 - 1].y);
               } else {
@@ -858,7 +895,9 @@ __global__ void __launch_bounds__(res_threads(ADJ), 1)
     // the words travel)
     if ((ADJ ? g_fold : vo != nullptr) && owner) {
 #pragma unroll 1
-      for (int r = er_lo * N; r < min(er_hi * N, Q.R); ++r) {
+      for (int q = er_lo * NJ; q < er_hi * NJ; ++q) {
+        const int r = q / NJ * N + h * NJ + q % NJ;
+        if (r >= Q.R) break;
         const int gi = (Q.gz0 + r) * pitch + Q.gx0 + ec * N, oi = r * L.Cp + ec * N;
         if (!ADJ) {
 #pragma unroll 1

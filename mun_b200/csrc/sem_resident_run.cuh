@@ -8,22 +8,23 @@ SolveIo solve_io(const sem_solve_t& s, const Workspace& ws, char* a);
 typedef void (*ResFn)(const SolveDev*, const int*, ResLay, unsigned long long*, unsigned, int, int, int, int, int);
 
 template <bool ADJ, bool STC>
-ResFn res_fn(int N) {
+ResFn res_fn(int N, int lpe) {
   switch (N) {
-    case 1: return sem_resident_kernel<1, ADJ, STC>;
-    case 2: return sem_resident_kernel<2, ADJ, STC>;
-    case 3: return sem_resident_kernel<3, ADJ, STC>;
-    case 4: return sem_resident_kernel<4, ADJ, STC>;
-    case 5: return sem_resident_kernel<5, ADJ, STC>;
-    case 6: return sem_resident_kernel<6, ADJ, STC>;
-    case 7: return sem_resident_kernel<7, ADJ, STC>;
+    case 1: return sem_resident_kernel<1, 1, ADJ, STC>;
+    case 2: return sem_resident_kernel<2, 1, ADJ, STC>;
+    case 3: return sem_resident_kernel<3, 1, ADJ, STC>;
+    case 4: return lpe == 2 ? sem_resident_kernel<4, 2, ADJ, STC> : sem_resident_kernel<4, 1, ADJ, STC>;
+    case 5: return sem_resident_kernel<5, 1, ADJ, STC>;
+    case 6: return sem_resident_kernel<6, 1, ADJ, STC>;
+    case 7: return sem_resident_kernel<7, 1, ADJ, STC>;
   }
   return nullptr;
 }
-ResFn res_kernel_for(int N, bool adj, bool stc) {
-  if (adj) return stc ? res_fn<true, true>(N) : res_fn<true, false>(N);
-  return stc ? res_fn<false, true>(N) : res_fn<false, false>(N);
+ResFn res_kernel_for(int N, int lpe, bool adj, bool stc) {
+  if (adj) return stc ? res_fn<true, true>(N, lpe) : res_fn<true, false>(N, lpe);
+  return stc ? res_fn<false, true>(N, lpe) : res_fn<false, false>(N, lpe);
 }
+int res_max_lanes(int N) { return N == 4 ? 2 : 1; }  // lanes per element
 
 // Receiver lists of the balanced tiling ntx x ntz of a plan (tiles from res_start).
 int get_res_lists(const sem_plan_s* p, int ntx, int ntz, sem_plan_s::ResLists* out) {
@@ -93,17 +94,23 @@ int get_res_lists(const sem_plan_s* p, int ntx, int ntz, sem_plan_s::ResLists* o
   return SEM_OK;
 }
 
-struct ResCounts { int nrec = 0, ninj = 0, nquad = 0, nterm = 0; };
+typedef sem_plan_s::ResCounts ResCounts;
+typedef sem_plan_s::ResTiling ResTiling;
+void take_max(ResCounts& a, const ResCounts& b) {
+  a.nrec = std::max(a.nrec, b.nrec); a.ninj = std::max(a.ninj, b.ninj);
+  a.nquad = std::max(a.nquad, b.nquad); a.nterm = std::max(a.nterm, b.nterm);
+}
 
-ResLay res_layout(int N, bool adj, bool stc, int exm, int ezm, const ResCounts& c) {
+ResLay res_layout(int N, int lpe, bool adj, bool stc, int exm, int ezm, const ResCounts& c) {
   ResLay L{};
   const int NP = N + 1;
-  auto odd4 = [](int v) { const int q = (v + 3) / 4; return 4 * (q | 1); };  // 128-bit rows of lanes spread over the banks
+  // rows of lanes spread over the banks: two lanes per element read rows two apart at once
+  auto pitch = [&](int v) { return lpe == 2 ? (v + 7) / 16 * 16 + 8 : 4 * ((v + 3) / 4 | 1); };
   L.Rm = ezm * N + 1;
   L.Cm = exm * N + 1;
   L.qx = exm + 1;
-  L.Wp = odd4((N == 4 ? 0 : 4) + N + (exm + 1) * N);
-  L.Cp = odd4((exm + 1) * N);
+  L.Wp = pitch((N == 4 ? 0 : 4) + N + (exm + 1) * N);
+  L.Cp = pitch((exm + 1) * N);
   const int rows = (ezm + 1) * N;  // one more element row: the mesh's last line of nodes starts it
   L.H = N + rows + 1;
   int o = 0;
@@ -136,32 +143,35 @@ ResLay res_layout(int N, bool adj, bool stc, int exm, int ezm, const ResCounts& 
 
 constexpr int kResSmem = 230400;  // dynamic shared bytes: one CTA per SM
 // Threads of a launch whose largest tile is exm x ezm elements (the lowest ezl high): lanes per
-// tile row, element rows per chunk, compute and receiver threads.
-struct ResShape { int sw, ezc, nc, nio; };
-bool res_shape(bool adj, int exm, int ezm, int ezl, int nrec, ResShape* h) {
+// tile row, element rows per chunk, compute and receiver threads; exchange words.
+struct ResShape { int sw, ezc, nc, nio, edge; };
+bool res_shape(int N, int lpe, bool adj, int exm, int ezm, int ezl, int nrec, ResShape* h) {
   const int ezr = std::max(ezm, ezl + 1);  // element rows, the mesh's last line of nodes counted as one
   h->nio = (int)round_up(std::max(nrec, 1), 32);
-  const int tmax = res_threads(adj) - h->nio;
+  h->edge = (exm + ezm) * N * (N + 1);
+  const int tmax = res_threads(lpe, adj) - h->nio;
   h->sw = 4;
-  while (h->sw < exm + 2) h->sw *= 2;
+  while (h->sw < (exm + 2) * lpe) h->sw *= 2;
   if (h->sw > 32 || tmax < 32) return false;
   h->ezc = (ezr + tmax / h->sw - 1) / (tmax / h->sw);
   h->nc = (int)round_up((long long)((ezr + h->ezc - 1) / h->ezc) * h->sw, 32);
   return true;
 }
-// Modelled cycles of one step: the exchange (send, 0.47 us between SMs, poll), then the warps'
-// work: per element and chunk the fp32 operations, at 1.95 cycles each for a warp alone on its
-// scheduler and 1.9 (adjoint 2.6: fewer warps) times the warps per scheduler beyond that.
-// Fitted to 100x50 meshes, order 4: a forward step of 25x25 tiles 11.0k cycles measured (11.1k
-// modelled), adjoint at 13x25 12.6k (12.3k), 4x2 tiles 3.7k / 4.5k (3.8k / 4.5k).  Two or three
-// smaller CTAs per SM, which hide one another's exchange, measured the same or slower (16
-// models, forward + adjoint: 18.1 us a step at best with one, 18.9 with two, 22.5 with three).
-double res_step_cost(int N, bool adj, const ResShape& h) {
+// Modelled cycles of one step: the exchange (0.47 us between SMs, poll, send, barrier; 1.2 a word),
+// then the warps' work: the fp32 operations of a lane, chunk by chunk, at 1.6 cycles (adjoint 1.7
+// with two lanes per element, 1.9 with one: fewer warps hide less) times the warps per scheduler.
+// Fitted to meshes of 20x10 to 200x100, order 4, to within 8 % (adjoint with two lanes: 14 %).
+// Two lanes per element halve a step's serial work, which decides small tiles (100x50 alone:
+// 1.84 us forward and 4.35 with the adjoint, 2.16 and 4.79 with one lane); one lane has no
+// swaps between them, which decides full SMs (128 of 100x50: 133 us a step, 142 with two).
+// Two or three smaller CTAs per SM, which hide one another's exchange, measured the same or
+// slower (16 of 100x50 with one lane: 18.1 us a step with one, 18.9 with two, 22.5 with three).
+double res_step_cost(int N, int lpe, bool adj, const ResShape& h) {
   const double NP = N + 1;
   const double el = adj ? 2 * N * (3 * NP * NP + 4 * NP) + 16 * N * N : 2 * N * (2 * NP * NP + 2 * NP) + 10 * N * N;
   const double carry = N * (NP * NP + 3 * NP) + (adj ? N * (NP + 2) : 0);
-  const double work = h.ezc * el + carry, warps = h.nc / 32.0;
-  return 2200.0 + work * std::max(1.95, (adj ? 2.6 : 1.9) * warps / 4.0);
+  const double fixed = lpe == 2 ? 2600.0 : adj ? 2300.0 : 2500.0, rate = !adj ? 1.6 : lpe == 2 ? 1.7 : 1.9;
+  return fixed + 1.2 * h.edge + rate * std::max(1.0, h.nc / 128.0) * (h.ezc * el + carry) / lpe;
 }
 bool res_fits(const ResLay& L) { return L.Wp <= 256 && L.H <= 256 && (long long)L.total * 4 <= kResSmem; }
 
@@ -196,66 +206,138 @@ ResCounts res_counts(const sem_plan_s* p, int ntx, int ntz) {
 }
 
 // Tiling of a plan into tiles of at most E elements that fit a CTA: the one with the least work
-// (tiles times modelled step); kept with the plan.  (0, 0): none.
-std::pair<int, int> res_tiling(const sem_plan_s* p, bool adj, int E) {
+// (tiles times modelled step); kept with the plan.  0 x 0: none.
+ResTiling res_tiling(const sem_plan_s* p, int lpe, bool adj, int E) {
   std::lock_guard<std::mutex> lk(p->mu);
-  const auto key = std::make_pair(adj, E);
+  const auto key = std::make_tuple(lpe, adj, E);
   auto it = p->res_tilings.find(key);
   if (it != p->res_tilings.end()) return it->second;
-  std::pair<int, int> best(0, 0);
+  ResTiling best;
   double best_c = -1.0;
   const bool stc = p->bnd_n > 0;
   for (int tx = 1; tx <= p->nelx; ++tx) {
     const int ex = (p->nelx + tx - 1) / tx;
     if (tx > 1 && ex == (p->nelx + tx - 2) / (tx - 1)) continue;  // no narrower than with one tile less
     const int ezm = E / ex;
-    if (ezm < 1 || ex > 30) continue;
+    if (ezm < 1 || (ex + 2) * lpe > 32) continue;
     const int tz = (p->nelz + ezm - 1) / ezm, ez = (p->nelz + tz - 1) / tz;
     ResShape h;
-    if (!res_shape(adj, ex, ez, p->nelz / tz, 1, &h)) continue;
-    const double c = (double)tx * tz * res_step_cost(p->npol, adj, h);
-    if (best_c >= 0.0 && c >= best_c) continue;
+    if (!res_shape(p->npol, lpe, adj, ex, ez, p->nelz / tz, 1, &h)) continue;
+    const double c = res_step_cost(p->npol, lpe, adj, h);
+    if (best_c >= 0.0 && tx * tz * c >= best_c) continue;
     const ResCounts cnt = res_counts(p, tx, tz);
-    if (!res_shape(adj, ex, ez, p->nelz / tz, std::max(cnt.nrec, cnt.ninj), &h) ||
-        !res_fits(res_layout(p->npol, adj, stc, ex, ez, cnt)))
+    if (!res_shape(p->npol, lpe, adj, ex, ez, p->nelz / tz, adj ? cnt.ninj : cnt.nrec, &h) ||
+        !res_fits(res_layout(p->npol, lpe, adj, stc, ex, ez, cnt)))
       continue;
-    best_c = c;
-    best = std::make_pair(tx, tz);
+    best.tx = tx; best.tz = tz;
+    best.n = cnt;
+    best_c = tx * tz * c;
   }
   p->res_tilings[key] = best;
   return best;
 }
 
-struct ResWave {
-  std::vector<int> idx;                        // solves
-  std::vector<std::pair<int, int>> tiles;      // their tilings
-  std::vector<int> k;                          // their checkpoint intervals
+// Waves of one kernel over a group of solves: each solve's tiling, and the solves (places in the
+// group) whose CTAs are resident at once.  A wave's launch shape is its largest tile's.
+struct ResPack {
+  int lpe = 0;
+  double cost = -1.0;  // modelled cycles; < 0: a solve does not fit
+  std::vector<ResTiling> tiles;
+  std::vector<std::vector<int>> waves;
+};
+struct ResGroup {
+  std::vector<int> idx, k;  // solves and their checkpoint intervals
+  ResPack fwd, adj;
 };
 
-int res_steps(const sem_solve_t& s, int k) {
-  const int nt = s.plan->nt;
-  if (!(s.flags & SEM_F_ADJOINT)) return nt;
-  const int nseg = (nt + k - 1) / k;
-  return nt + k * (nseg - 1);
+// For each tile capacity, pack the solves (in order) into waves and keep the capacity, and the
+// lanes per element, with the smallest modelled time.  steps: time steps of each solve's launches.
+ResPack res_pack(const sem_solve_t* sv, const std::vector<int>& idx, const std::vector<int>& steps, bool adj, int sms) {
+  const int n = (int)idx.size(), N = sv[idx[0]].plan->npol;
+  std::vector<const sem_plan_s*> plans;
+  std::vector<int> pl(n);
+  for (int j = 0; j < n; ++j) {
+    const auto f = std::find(plans.begin(), plans.end(), sv[idx[j]].plan);
+    pl[j] = (int)(f - plans.begin());
+    if (f == plans.end()) plans.push_back(sv[idx[j]].plan);
+  }
+  const bool stc = plans[0]->bnd_n > 0;
+  ResPack best;
+  std::vector<ResTiling> tl(plans.size()), last;
+  std::vector<int> first;
+  for (int lpe = 1; lpe <= res_max_lanes(N); ++lpe) {
+    last.clear();
+    for (double Ed = 8.0; Ed < 1200.0; Ed *= 1.15) {
+      bool ok = true, same = !last.empty();
+      for (size_t q = 0; q < plans.size() && ok; ++q) {
+        tl[q] = res_tiling(plans[q], lpe, adj, (int)Ed);
+        ok = tl[q].tx > 0 && (long long)tl[q].tx * tl[q].tz <= sms;
+        same = same && tl[q].tx == last[q].tx && tl[q].tz == last[q].tz;
+      }
+      if (!ok || same) continue;
+      last = tl;
+      first.clear();
+      double cost = 0.0, step = 0.0;
+      int used = 0, nt = 0, exm = 0, ezm = 0, ezl = 0;
+      ResCounts cnt;
+      for (int j = 0; j < n; ++j) {
+        const ResTiling& t = tl[pl[j]];
+        const sem_plan_s* p = plans[pl[j]];
+        const int ex = (p->nelx + t.tx - 1) / t.tx, ez = (p->nelz + t.tz - 1) / t.tz, el = p->nelz / t.tz;
+        ResCounts c = cnt;
+        take_max(c, t.n);
+        ResShape h;
+        bool fits = j > 0 && used + t.tx * t.tz <= sms;
+        if (fits) {
+          const int x = std::max(ex, exm), z = std::max(ez, ezm);
+          fits = res_shape(N, lpe, adj, x, z, std::max(el, ezl), adj ? c.ninj : c.nrec, &h) &&
+                 res_fits(res_layout(N, lpe, adj, stc, x, z, c));
+        }
+        if (!fits) {  // the next wave
+          cost += step * nt;
+          first.push_back(j);
+          used = nt = exm = ezm = ezl = 0;
+          c = t.n;
+          res_shape(N, lpe, adj, ex, ez, el, adj ? c.ninj : c.nrec, &h);
+        }
+        cnt = c;
+        used += t.tx * t.tz;
+        exm = std::max(exm, ex); ezm = std::max(ezm, ez); ezl = std::max(ezl, el);
+        step = res_step_cost(N, lpe, adj, h);
+        nt = std::max(nt, steps[j]);
+      }
+      cost += step * nt;
+      if (best.cost >= 0.0 && cost >= best.cost) continue;
+      best.cost = cost;
+      best.lpe = lpe;
+      best.tiles.resize(n);
+      for (int j = 0; j < n; ++j) best.tiles[j] = tl[pl[j]];
+      best.waves.clear();
+      for (size_t w = 0; w < first.size(); ++w) {
+        best.waves.emplace_back();
+        for (int j = first[w]; j < (w + 1 < first.size() ? first[w + 1] : n); ++j) best.waves.back().push_back(j);
+      }
+    }
+  }
+  return best;
 }
 
-// Waves of one class of solves (same order, boundary mode, forward-only or not): for each tile
-// capacity, pack the solves (longest first) into waves whose CTAs are resident at once and
-// whose workspaces fit the budget, and keep the capacity with the smallest modelled time.
+// Groups of one class of solves (same order, boundary mode, forward-only or not), longest first:
+// each group's workspaces fit the budget.  Forward and adjoint launches have waves of their own:
+// the forward kernel needs less room per element, so its waves hold more solves (128 models of
+// 100x50, forward and adjoint: 146 us a step when both had the adjoint's tiles, 132 now).
 // Empty when a solve fits no way.
-std::vector<ResWave> res_plan(const sem_solve_t* sv, const std::vector<int>& cls, int sms, long long budget) {
-  const sem_plan_s* p0 = sv[cls[0]].plan;
-  const int N = p0->npol;
+std::vector<ResGroup> res_plan(const sem_solve_t* sv, const std::vector<int>& cls, int sms, long long budget) {
   const bool adj = sv[cls[0]].flags & SEM_F_ADJOINT;
   std::vector<int> ord(cls);
   std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
     return (long long)sv[a].plan->nt * 64 + sv[a].plan->npoints / 4096 > (long long)sv[b].plan->nt * 64 + sv[b].plan->npoints / 4096;
   });
-  // checkpoint interval and bytes of each solve by itself
-  std::vector<int> kk(ord.size());
-  std::vector<long long> bytes(ord.size());
-  for (size_t j = 0; j < ord.size(); ++j) {
-    const sem_solve_t& s = sv[ord[j]];
+  std::vector<ResGroup> groups;
+  long long mem = 0;
+  for (int i : ord) {
+    // checkpoint interval and bytes of the solve by itself
+    const sem_solve_t& s = sv[i];
     int ns, k = 2;
     if (adj) {
       k = std::max(2, std::min(s.ckpt_k > 0 ? (int)s.ckpt_k : s.plan->nt, s.plan->nt));
@@ -268,90 +350,91 @@ std::vector<ResWave> res_plan(const sem_solve_t* sv, const std::vector<int>& cls
         k = lo;
       }
     }
-    kk[j] = k;
-    bytes[j] = layout(s.plan, s.flags, k, &ns).bytes;
-  }
-  std::vector<ResWave> best;
-  double best_cost = -1.0;
-  for (double Ed = 8.0; Ed < 1200.0; Ed *= 1.15) {
-    const int E = (int)Ed;
-    std::vector<ResWave> waves;
-    double cost = 0.0;
-    bool ok = true;
-    long long used = 0, mem = 0;
-    double wave_step = 0.0;
-    int wave_nt = 0;
-    auto close = [&]() { cost += wave_step * wave_nt; used = mem = 0; wave_step = 0.0; wave_nt = 0; };
-    for (size_t j = 0; j < ord.size() && ok; ++j) {
-      const sem_plan_s* p = sv[ord[j]].plan;
-      const std::pair<int, int> tile = res_tiling(p, adj, E);
-      const int tx = tile.first, tz = tile.second;
-      if (!tx || (long long)tx * tz > sms) { ok = false; break; }
-      if (waves.empty() || used + (long long)tx * tz > sms || mem + bytes[j] > budget) {
-        if (!waves.empty()) close();
-        waves.emplace_back();
-      }
-      ResWave& w = waves.back();
-      w.idx.push_back(ord[j]);
-      w.tiles.push_back(tile);
-      w.k.push_back(kk[j]);
-      used += (long long)tx * tz;
-      mem += bytes[j];
-      ResShape h;
-      const int ex = (p->nelx + tx - 1) / tx, ez = (p->nelz + tz - 1) / tz;
-      double c = 0.0;
-      for (int a = 0; a <= (adj ? 1 : 0); ++a) {
-        if (!res_shape(a, ex, ez, p->nelz / tz, 32, &h)) { ok = false; break; }
-        c += res_step_cost(N, a, h);
-      }
-      wave_step = std::max(wave_step, c);
-      wave_nt = std::max(wave_nt, res_steps(sv[ord[j]], kk[j]));
-      if (best_cost >= 0.0 && cost > best_cost) ok = false;
+    const long long bytes = layout(s.plan, s.flags, k, &ns).bytes;
+    if (groups.empty() || mem + bytes > budget) {
+      groups.emplace_back();
+      mem = 0;
     }
-    if (!ok) continue;
-    close();
-    if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = waves; }
+    groups.back().idx.push_back(i);
+    groups.back().k.push_back(k);
+    mem += bytes;
   }
-  return best;
+  for (ResGroup& g : groups) {
+    std::vector<int> nf, na;
+    for (size_t j = 0; j < g.idx.size(); ++j) {
+      const int nt = sv[g.idx[j]].plan->nt, k = g.k[j];
+      nf.push_back(nt + (adj ? k * ((nt + k - 1) / k - 1) : 0));
+      na.push_back(nt);
+    }
+    g.fwd = res_pack(sv, g.idx, nf, false, sms);
+    if (g.fwd.cost < 0.0) return {};
+    if (!adj) continue;
+    g.adj = res_pack(sv, g.idx, na, true, sms);
+    if (g.adj.cost < 0.0) return {};
+  }
+  return groups;
 }
 
-// One wave: set-up, forward launch, (replay and) adjoint launches, outputs.
-// SEM_ERR_UNSUPPORTED without a message when the wave cannot run this way (nothing launched).
-int run_res_wave(sem_batch_t* b, const sem_solve_t* sv, const ResWave& w, int sms, cudaStream_t stream) {
+// One launch shape: a wave of one kernel.
+struct ResWave {
+  ResFn fn;
+  ResLay L;
+  ResShape h;
+  int ncta, cta0;           // CTAs, and where their list starts
+  const std::vector<int>* solves;
+};
+
+// One group: set-up, forward launches, (replay and) adjoint launches, outputs.
+// SEM_ERR_UNSUPPORTED without a message when the group cannot run this way (nothing launched).
+int run_res_group(sem_batch_t* b, const sem_solve_t* sv, const ResGroup& w, int sms, cudaStream_t stream) {
   const int n = (int)w.idx.size();
   const sem_plan_s* p0 = sv[w.idx[0]].plan;
   const int N = p0->npol;
   const bool adj = sv[w.idx[0]].flags & SEM_F_ADJOINT, stc = p0->bnd_n > 0;
-  int exm = 1, ezm = 1;
-  ResCounts c;
-  std::vector<sem_plan_s::ResLists> lists(n);
-  long long ncta = 0;
-  int ezl = 1;
-  for (int j = 0; j < n; ++j) {
-    const sem_plan_s* p = sv[w.idx[j]].plan;
-    const int tx = w.tiles[j].first, tz = w.tiles[j].second;
-    if (int rc = get_res_lists(p, tx, tz, &lists[j])) return rc;
-    c.nrec = std::max(c.nrec, lists[j].nrec); c.ninj = std::max(c.ninj, lists[j].ninj);
-    c.nquad = std::max(c.nquad, lists[j].nquad); c.nterm = std::max(c.nterm, lists[j].nterm);
-    exm = std::max(exm, (p->nelx + tx - 1) / tx); ezm = std::max(ezm, (p->nelz + tz - 1) / tz);
-    ezl = std::max(ezl, p->nelz / tz);
-    ncta += (long long)tx * tz;
-  }
-  const ResLay Lf = res_layout(N, false, stc, exm, ezm, c), La = adj ? res_layout(N, true, stc, exm, ezm, c) : Lf;
-  ResShape hf, ha;
-  if (!res_shape(false, exm, ezm, ezl, c.nrec, &hf) || !res_shape(true, exm, ezm, ezl, c.ninj, &ha))
-    return SEM_ERR_UNSUPPORTED;
-  ResFn ff = res_kernel_for(N, false, stc), fa = adj ? res_kernel_for(N, true, stc) : nullptr;
+  // ---- launch shapes of the forward and adjoint waves
+  std::vector<sem_plan_s::ResLists> lists[2];
+  std::vector<ResWave> waves[2];
+  std::vector<int> wave_of(n), base[2];
+  long long ll_words = 0;
+  int cta0 = 0;
   for (int q = 0; q < (adj ? 2 : 1); ++q) {
-    ResFn fn = q ? fa : ff;
-    const ResLay& L = q ? La : Lf;
-    const int T = q ? ha.nc + ha.nio : hf.nc + hf.nio;
-    int nb = 0;
-    if (!res_fits(L) || raise_smem_limit((const void*)fn, (size_t)L.total * 4) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, T, (size_t)L.total * 4) != cudaSuccess ||
-        (long long)nb * sms < ncta) {
-      cudaGetLastError();
-      return SEM_ERR_UNSUPPORTED;
+    const ResPack& pk = q ? w.adj : w.fwd;
+    lists[q].resize(n);
+    base[q].resize(n);
+    for (const std::vector<int>& wv : pk.waves) {
+      ResWave v{};
+      ResCounts c;
+      int exm = 1, ezm = 1, ezl = 1;
+      for (int j : wv) {
+        const sem_plan_s* p = sv[w.idx[j]].plan;
+        const int tx = pk.tiles[j].tx, tz = pk.tiles[j].tz;
+        sem_plan_s::ResLists& l = lists[q][j];
+        if (int rc = get_res_lists(p, tx, tz, &l)) return rc;
+        c.nrec = std::max(c.nrec, l.nrec); c.ninj = std::max(c.ninj, l.ninj);
+        c.nquad = std::max(c.nquad, l.nquad); c.nterm = std::max(c.nterm, l.nterm);
+        exm = std::max(exm, (p->nelx + tx - 1) / tx); ezm = std::max(ezm, (p->nelz + tz - 1) / tz);
+        ezl = std::max(ezl, p->nelz / tz);
+        base[q][j] = v.ncta;
+        v.ncta += tx * tz;
+      }
+      v.cta0 = cta0;
+      cta0 += v.ncta;
+      v.solves = &wv;
+      v.L = res_layout(N, pk.lpe, q, stc, exm, ezm, c);
+      v.fn = res_kernel_for(N, pk.lpe, q, stc);
+      if (!res_shape(N, pk.lpe, q, exm, ezm, ezl, q ? c.ninj : c.nrec, &v.h)) return SEM_ERR_UNSUPPORTED;
+      int nb = 0;
+      if (!res_fits(v.L) || raise_smem_limit((const void*)v.fn, (size_t)v.L.total * 4) != cudaSuccess ||
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, v.fn, v.h.nc + v.h.nio, (size_t)v.L.total * 4) != cudaSuccess ||
+          (long long)nb * sms < v.ncta) {
+        cudaGetLastError();
+        return SEM_ERR_UNSUPPORTED;
+      }
+      ll_words = std::max(ll_words, (long long)v.ncta * kResSlots * v.L.llw);
+      if (q)
+        for (int j : wv) wave_of[j] = (int)waves[q].size();
+      else { b->last_tile_ex = exm; b->last_tile_ez = ezm; }
+      waves[q].push_back(v);
     }
   }
 
@@ -359,14 +442,12 @@ int run_res_wave(sem_batch_t* b, const sem_solve_t* sv, const ResWave& w, int sm
   std::vector<Workspace> ws(n);
   std::vector<int> nseg(n);
   long long total = 0;
-  int max_prog = 0, max_seg = 1;
+  int max_seg = 1;
   for (int j = 0; j < n; ++j) {
     const sem_solve_t& s = sv[w.idx[j]];
     ws[j] = layout(s.plan, s.flags, w.k[j], &nseg[j]);
     total += ws[j].bytes;
     max_seg = std::max(max_seg, nseg[j]);
-    const int nt = s.plan->nt;
-    max_prog = std::max(max_prog, nt + ((s.flags & SEM_F_SHIFT) ? 1 : 0) + (adj ? 1 + nt + w.k[j] * (nseg[j] - 1) : 0));
   }
   if (total > b->arena_bytes) {
     cudaFree(b->arena);
@@ -383,8 +464,9 @@ int run_res_wave(sem_batch_t* b, const sem_solve_t* sv, const ResWave& w, int sm
     b->tmaps_cap = n;
   }
   b->h_tmaps.resize(n);
-  b->h_solves.assign(n, SolveDev{});
-  b->h_cta.clear();
+  const int nq = adj ? 2 : 1;  // descriptors: the forward waves', then the adjoint waves'
+  b->h_solves.assign((size_t)n * nq, SolveDev{});
+  b->h_cta.resize(cta0);
   b->h_io.clear();
   long long off = 0, max_pts = 1;
   for (int j = 0; j < n; ++j) {
@@ -393,9 +475,9 @@ int run_res_wave(sem_batch_t* b, const sem_solve_t* sv, const ResWave& w, int sm
     char* a = b->arena + off;
     SolveDev& d = b->h_solves[j];
     d.nelx = p->nelx; d.nelz = p->nelz; d.nxg = p->nxg; d.nzg = p->nzg; d.pitch = p->pitch;
-    d.tiles_x = w.tiles[j].first; d.tiles_z = w.tiles[j].second;
+    d.tiles_x = w.fwd.tiles[j].tx; d.tiles_z = w.fwd.tiles[j].tz;
     d.zchunk = p->nelz;
-    d.tile_base = (int)b->h_cta.size();
+    d.tile_base = base[0][j];
     d.nt = p->nt; d.k = w.k[j]; d.nseg = nseg[j]; d.flags = s.flags; d.start_tick = 0;
     d.it0 = s.it0; d.it1 = s.it1; d.decim = s.decim;
     d.src_gx = p->src_gx; d.src_gz = p->src_gz; d.nrec = p->nrec;
@@ -410,15 +492,13 @@ int run_res_wave(sem_batch_t* b, const sem_solve_t* sv, const ResWave& w, int sm
       d.Mu = (float*)(a + ws[j].Mu);
       d.grad = (float*)(a + ws[j].grad);
       d.grad64 = (double*)(a + ws[j].grad64);
-      if (int rc = encode_band_map(&b->h_tmaps[j], a, p, field_slots(ws[j], p, true), La.Wp, La.H)) return rc;
+      const ResLay& L = waves[1][wave_of[j]].L;
+      if (int rc = encode_band_map(&b->h_tmaps[j], a, p, field_slots(ws[j], p, true), L.Wp, L.H)) return rc;
       d.tmap = b->d_tmaps + j;
     }
     d.D = p->D; d.beta = p->beta; d.tx = p->tx; d.tz = p->tz; d.src_term = p->src_term;
     d.rec_base = p->rec_base; d.rec_w = p->rec_w;
-    d.rec_tile_off = lists[j].l.rec_off; d.rec_tile_ids = lists[j].l.rec_ids;
-    d.inj_tile_off = lists[j].l.inj_off; d.inj_tile_ids = lists[j].l.inj_ids;
-    d.iq_off = lists[j].iq_off; d.iq_pos = lists[j].iq_pos; d.iterm_off = lists[j].iterm_off;
-    d.iterm = lists[j].iterm; d.iterm_w = lists[j].iterm_w;
+    d.rec_tile_off = lists[0][j].l.rec_off; d.rec_tile_ids = lists[0][j].l.rec_ids;
     d.rec_out = s.rec_out; d.yobs = s.y_obs;
     d.misfit = (double*)(a + ws[j].misfit);
     d.rmax = d.misfit + p->nrec;
@@ -428,17 +508,33 @@ int run_res_wave(sem_batch_t* b, const sem_solve_t* sv, const ResWave& w, int sm
     d.bnd_n = p->bnd_n; d.bnd_pitch = bnd_pitch_of(p);
     d.bnd_coef = p->bnd_n ? (const float*)(a + ws[j].bnd_coef) : nullptr;
     d.bnd_hist = ws[j].bnd_hist >= 0 ? (float*)(a + ws[j].bnd_hist) : nullptr;
-    b->h_cta.insert(b->h_cta.end(), d.tiles_x * d.tiles_z, j);
+    if (adj) {
+      SolveDev& e = b->h_solves[n + j];
+      const sem_plan_s::ResLists& l = lists[1][j];
+      e = d;
+      e.tiles_x = w.adj.tiles[j].tx; e.tiles_z = w.adj.tiles[j].tz;
+      e.tile_base = base[1][j];
+      e.rec_tile_off = l.l.rec_off; e.rec_tile_ids = l.l.rec_ids;
+      e.inj_tile_off = l.l.inj_off; e.inj_tile_ids = l.l.inj_ids;
+      e.iq_off = l.iq_off; e.iq_pos = l.iq_pos; e.iterm_off = l.iterm_off;
+      e.iterm = l.iterm; e.iterm_w = l.iterm_w;
+    }
     b->h_io.push_back(solve_io(s, ws[j], a));
     max_pts = std::max(max_pts, (long long)p->npoints);
     off += ws[j].bytes;
   }
-  if (n > b->solves_cap) {
+  for (int q = 0; q < nq; ++q)
+    for (const ResWave& v : waves[q])
+      for (int j : *v.solves) {
+        const SolveDev& d = b->h_solves[q * n + j];
+        std::fill_n(b->h_cta.begin() + v.cta0 + d.tile_base, d.tiles_x * d.tiles_z, q * n + j);
+      }
+  if (n * nq > b->solves_cap) {
     cudaFree(b->d_solves);
     b->d_solves = nullptr;
     b->solves_cap = 0;
-    CUDA_TRY(cudaMalloc((void**)&b->d_solves, sizeof(SolveDev) * n));
-    b->solves_cap = n;
+    CUDA_TRY(cudaMalloc((void**)&b->d_solves, sizeof(SolveDev) * n * nq));
+    b->solves_cap = n * nq;
   }
   if ((long long)b->h_cta.size() > b->cta_cap) {
     cudaFree(b->d_cta);
@@ -454,7 +550,7 @@ int run_res_wave(sem_batch_t* b, const sem_solve_t* sv, const ResWave& w, int sm
     CUDA_TRY(cudaMalloc((void**)&b->d_io, sizeof(SolveIo) * n));
     b->io_cap = n;
   }
-  const long long ll_bytes = ncta * kResSlots * (long long)std::max(Lf.llw, La.llw) * 8;
+  const long long ll_bytes = ll_words * 8;
   if (ll_bytes > b->ll_cap) {
     cudaFree(b->d_ll);
     b->d_ll = nullptr;
@@ -464,7 +560,7 @@ int run_res_wave(sem_batch_t* b, const sem_solve_t* sv, const ResWave& w, int sm
     CUDA_TRY(cudaMemsetAsync(b->d_ll, 0, ll_bytes, stream));
     b->ll_tag = 0;
   }
-  CUDA_TRY(cudaMemcpyAsync(b->d_solves, b->h_solves.data(), sizeof(SolveDev) * n, cudaMemcpyHostToDevice, stream));
+  CUDA_TRY(cudaMemcpyAsync(b->d_solves, b->h_solves.data(), sizeof(SolveDev) * n * nq, cudaMemcpyHostToDevice, stream));
   if (adj)
     CUDA_TRY(cudaMemcpyAsync(b->d_tmaps, b->h_tmaps.data(), sizeof(CUtensorMap) * n, cudaMemcpyHostToDevice, stream));
   CUDA_TRY(cudaMemcpyAsync(b->d_cta, b->h_cta.data(), sizeof(int) * b->h_cta.size(), cudaMemcpyHostToDevice, stream));
@@ -482,35 +578,34 @@ int run_res_wave(sem_batch_t* b, const sem_solve_t* sv, const ResWave& w, int sm
   }
   CUDA_TRY(cudaEventRecord(b->tick_ev[b->tick_ev_used], stream));
   auto launch = [&](int kind, int idx) -> int {
-    int steps = 0;
-    for (int j = 0; j < n; ++j) {
-      const SolveDev& d = b->h_solves[j];
-      int seg, t0, t1;
-      if ((kind == RES_FWD || (d.flags & F_ADJ)) && res_range(kind, idx, d.nt, d.k, d.nseg, d.it0, d.it1, seg, t0, t1))
-        steps = std::max(steps, t1 - t0);
+    const int q = kind == RES_ADJ;
+    for (const ResWave& v : waves[q]) {
+      int steps = 0;
+      for (int j : *v.solves) {
+        const SolveDev& d = b->h_solves[j];
+        int seg, t0, t1;
+        if (res_range(kind, idx, d.nt, d.k, d.nseg, d.it0, d.it1, seg, t0, t1)) steps = std::max(steps, t1 - t0);
+      }
+      if (steps == 0) continue;
+      if (b->ll_tag > 0xf0000000u - (unsigned)steps) {
+        CUDA_TRY(cudaMemsetAsync(b->d_ll, 0, b->ll_cap, stream));
+        b->ll_tag = 0;
+      }
+      cudaLaunchConfig_t lc = {};
+      lc.gridDim = dim3((unsigned)v.ncta);
+      lc.blockDim = dim3((unsigned)(v.h.nc + v.h.nio));
+      lc.dynamicSmemBytes = (size_t)v.L.total * 4;
+      lc.stream = stream;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeCooperative;
+      at[0].val.cooperative = 1;
+      lc.attrs = at;
+      lc.numAttrs = 1;
+      CUDA_TRY(cudaLaunchKernelEx(&lc, v.fn, (const SolveDev*)b->d_solves, (const int*)b->d_cta + v.cta0, v.L, b->d_ll,
+                                  b->ll_tag, kind, idx, v.h.nc, v.h.sw, v.h.ezc));
+      b->ll_tag += (unsigned)steps + 2;
+      b->last_launches++;
     }
-    if (steps == 0) return SEM_OK;
-    if (b->ll_tag > 0xf0000000u - (unsigned)steps) {
-      CUDA_TRY(cudaMemsetAsync(b->d_ll, 0, b->ll_cap, stream));
-      b->ll_tag = 0;
-    }
-    const bool a = kind == RES_ADJ;
-    const ResLay& L = a ? La : Lf;
-    const ResShape& h = a ? ha : hf;
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)ncta);
-    lc.blockDim = dim3((unsigned)(h.nc + h.nio));
-    lc.dynamicSmemBytes = (size_t)L.total * 4;
-    lc.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    CUDA_TRY(cudaLaunchKernelEx(&lc, a ? fa : ff, (const SolveDev*)b->d_solves, (const int*)b->d_cta, L, b->d_ll,
-                                b->ll_tag, kind, idx, h.nc, h.sw, h.ezc));
-    b->ll_tag += (unsigned)steps + 2;
-    b->last_launches++;
     return SEM_OK;
   };
   int rc = launch(RES_FWD, 0);
@@ -521,14 +616,22 @@ int run_res_wave(sem_batch_t* b, const sem_solve_t* sv, const ResWave& w, int sm
   if (rc) return rc;
   CUDA_TRY(cudaEventRecord(b->tick_ev[b->tick_ev_used + 1], stream));
   b->tick_ev_used += 2;
-  b->last_ticks += max_prog;
+  for (int q = 0; q < nq; ++q)
+    for (const ResWave& v : waves[q]) {
+      int prog = 0;
+      for (int j : *v.solves) {
+        const SolveDev& d = b->h_solves[j];
+        prog = std::max(prog, q ? 1 + d.nt : d.nt + ((d.flags & F_SHIFT) ? 1 : 0) + (adj ? d.k * (d.nseg - 1) : 0));
+      }
+      b->last_ticks += prog;
+    }
   for (int s0 = 0; s0 < n; s0 += 65535)
     batch_output_kernel<<<dim3(io_bx, (unsigned)std::min(65535, n - s0)), 256, 0, stream>>>(b->d_io, s0);
   b->last_launches++;
   CUDA_TRY(cudaGetLastError());
   b->last_kernel = 5;
-  b->last_tile_ex = exm; b->last_tile_ez = ezm; b->last_zchunk = 0;
-  b->last_groups++;
+  b->last_zchunk = 0;
+  b->last_groups += (int)std::max(waves[0].size(), waves[1].size());
   return SEM_OK;
 }
 
@@ -541,11 +644,11 @@ int run_resident(sem_batch_t* b, const sem_solve_t* sv, int n, long long budget,
   for (int i = 0; i < n; ++i)
     classes[std::make_tuple(sv[i].plan->npol, sv[i].plan->bnd_n > 0, (sv[i].flags & SEM_F_ADJOINT) != 0)].push_back(i);
   for (auto& kv : classes) {
-    const std::vector<ResWave> waves = res_plan(sv, kv.second, sms, budget);
-    if (waves.empty()) { rest->insert(rest->end(), kv.second.begin(), kv.second.end()); continue; }
-    for (const ResWave& w : waves) {
-      const int rc = run_res_wave(b, sv, w, sms, stream);
-      if (rc == SEM_ERR_UNSUPPORTED) rest->insert(rest->end(), w.idx.begin(), w.idx.end());
+    const std::vector<ResGroup> groups = res_plan(sv, kv.second, sms, budget);
+    if (groups.empty()) { rest->insert(rest->end(), kv.second.begin(), kv.second.end()); continue; }
+    for (const ResGroup& g : groups) {
+      const int rc = run_res_group(b, sv, g, sms, stream);
+      if (rc == SEM_ERR_UNSUPPORTED) rest->insert(rest->end(), g.idx.begin(), g.idx.end());
       else if (rc) return rc;
     }
   }

@@ -4,18 +4,17 @@ from; every owned node is advanced by exactly one thread; every access lies insi
 import pytest
 
 
-def odd4(v):
-    q = (v + 3) // 4
-    return 4 * (q | 1)
+def pitch(lpe, v):
+    return (v + 7) // 16 * 16 + 8 if lpe == 2 else 4 * ((v + 3) // 4 | 1)
 
 
 class Layout:
     """The fields of ResLay that index arithmetic uses."""
 
-    def __init__(self, N, exm, ezm):
+    def __init__(self, N, lpe, exm, ezm):
         self.N, self.Rm, self.Cm, self.qx = N, ezm * N + 1, exm * N + 1, exm + 1
-        self.Wp = odd4((0 if N == 4 else 4) + N + (exm + 1) * N)
-        self.Cp = odd4((exm + 1) * N)
+        self.Wp = pitch(lpe, (0 if N == 4 else 4) + N + (exm + 1) * N)
+        self.Cp = pitch(lpe, (exm + 1) * N)
         self.rows = (ezm + 1) * N
         self.H = N + self.rows + 1
         self.t = self.Rm * N
@@ -75,12 +74,13 @@ def sends(T, L, t, ntx):
                     yield t - ntx - 1, L.c, r, 0
 
 
-@pytest.mark.parametrize("N,nelx,nelz,ntx,ntz", [
-    (1, 7, 5, 3, 2), (2, 9, 4, 4, 4), (3, 11, 7, 3, 3), (4, 10, 6, 10, 6), (4, 13, 9, 4, 3), (4, 5, 3, 1, 1),
-    (4, 8, 8, 1, 5), (5, 7, 9, 3, 2), (6, 5, 5, 2, 3), (7, 4, 4, 3, 2)])
-def test_exchange_and_bounds(N, nelx, nelz, ntx, ntz):
+@pytest.mark.parametrize("N,nelx,nelz,ntx,ntz,lpe", [
+    (1, 7, 5, 3, 2, 1), (2, 9, 4, 4, 4, 1), (3, 11, 7, 3, 3, 1), (4, 10, 6, 10, 6, 1), (4, 10, 6, 10, 6, 2),
+    (4, 13, 9, 4, 3, 1), (4, 13, 9, 4, 3, 2), (4, 5, 3, 1, 1, 2), (4, 14, 3, 1, 1, 2), (4, 30, 3, 1, 1, 1),
+    (4, 8, 8, 1, 5, 1), (4, 8, 8, 1, 5, 2), (5, 7, 9, 3, 2, 1), (6, 5, 5, 2, 3, 1), (7, 4, 4, 3, 2, 1)])
+def test_exchange_and_bounds(N, nelx, nelz, ntx, ntz, lpe):
     exm, ezm = -(-nelx // ntx), -(-nelz // ntz)
-    L = Layout(N, exm, ezm)
+    L = Layout(N, lpe, exm, ezm)
     tiles = [Tile(N, nelx, nelz, ntx, ntz, t) for t in range(ntx * ntz)]
     assert sum(T.R * T.C for T in tiles) == (nelx * N + 1) * (nelz * N + 1)
     sent = {}
@@ -100,7 +100,8 @@ def test_exchange_and_bounds(N, nelx, nelz, ntx, ntz):
     assert wanted == set(sent)
     # lanes: every owned node is advanced by exactly one thread; reads stay inside the arrays
     sw = 4
-    while sw < exm + 2:
+    nj = N // lpe
+    while sw < (exm + 2) * lpe:
         sw *= 2
     for ezc in (1, 2, 3):
         for T in tiles:
@@ -111,21 +112,27 @@ def test_exchange_and_bounds(N, nelx, nelz, ntx, ntz):
                 first = min(lo, ez1 - 1)
                 assert N + first * N < L.H and (not (lo < hi and (lo > 0 or T.ht)) or first * N >= 0)
                 for sl in range(sw):
-                    ec = min(sl - 1, T.EX)
-                    full = 1 <= sl <= T.EX
-                    owner = full or (sl == T.EX + 1 and not T.hr)
+                    el, h = sl // lpe, sl % lpe
+                    ec = min(el - 1, T.EX)
+                    full = 1 <= el <= T.EX
+                    owner = full or (el == T.EX + 1 and not T.hr)
                     col = T.off + N + ec * N
                     assert col >= 0 and col + N + (N & 1) <= L.Wp
-                    assert not full or sl + 1 < sw  # the next lane holds the nodes on the right
+                    assert not full or sl + lpe < sw  # the next lane holds the nodes on the right
                     for er in range(lo, lo + ezc):
                         e_ = min(er, ez1 - 1)
                         assert N + e_ * N + N < L.H and e_ * N + N <= L.rows
                         assert not owner or (ec + 1) * N <= L.Cp and ec < L.qx
                         if owner and er < hi:
-                            for j in range(1 if e_ == T.EZ else N):
+                            for j in range(nj):
+                                r = e_ * N + h * nj + j
+                                if e_ == T.EZ and r > T.EZ * N:
+                                    continue
                                 for i in range(N if full else 1):
-                                    assert (e_ * N + j, ec * N + i) not in seen
-                                    seen.add((e_ * N + j, ec * N + i))
+                                    assert (r, ec * N + i) not in seen
+                                    seen.add((r, ec * N + i))
+                                    # the warp that sends a node's exchange words is the one that advances it
+                                    assert ch * sw + (ec + 1) * lpe + (r % N) // nj == ch * sw + sl
             assert seen == {(r, c) for r in range(T.R) for c in range(T.C)}
             # receivers' elements, the corner node included, lie inside the region
             assert N + (T.EZ - 1) * N + N < L.H and T.off + N + (T.EX - 1) * N + N < L.Wp
