@@ -23,12 +23,19 @@
 //
 // Threads.  A compute thread owns a column of elements, or of their halves: lane by lane the
 // elements of a tile row, stepping down the element rows of its chunk.  All lines of an element
-// are evaluated in registers; the carry into the element below stays in registers, the carry into the right
-// neighbour goes by shuffle, and the first lane of a row is the left halo element, evaluated
-// for its carry only.  A chunk starts with the z-lines of the element row above it, for their
-// carry.  Nodes are advanced into the other of two buffers and each warp sends its own edge
-// nodes, so a step needs one CTA barrier, when the halo words have arrived.  A few threads beyond the
-// compute threads read out the receivers and form the adjoint source meanwhile.
+// are evaluated in registers; the carry into the element below stays in registers, the carry into
+// the right neighbour goes by shuffle, and the first lane of a row is the left halo element,
+// evaluated for its carry only.  A chunk starts with the z-lines of the element row above it, for
+// their carry.  Nodes are advanced into the other of two buffers and each warp sends its own edge
+// nodes, so a step needs one CTA barrier, when the halo words have arrived.  A few threads beyond
+// the compute threads read out the receivers and form the adjoint source meanwhile.
+//
+// Large adjoint tiles (VG).  With displacement (two buffers), history (two), c^2, increment and
+// partial gradient on chip an SM holds about 300 elements of order 4, so a 400x200 mesh's adjoint
+// does not fit the GPU.  Increment and partial gradient are read and written once a step by the
+// thread that owns them: kept in the solve's fields they cost 16 bytes a node and step of L2
+// traffic, in flight during the x-lines, and 575 elements fit (forward + adjoint 15.7 us a step;
+// strips 27.7).  Where the tiles fit anyway, keeping them on chip is as fast or faster.
 //
 // Arithmetic.  Per node the operations and roundings of the tile and strip kernels, in the
 // same order: results are bitwise equal to theirs.
@@ -68,6 +75,27 @@ __device__ __forceinline__ unsigned long long ll_load(const unsigned long long* 
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
+}
+
+// Exchange words' table entries.  In: place in this CTA's slot and region index.  Out: place among
+// the words of the tile above on the left (and on from it) and region index.  Two ints; in the
+// kernels that need the room one: 16 bits region index, two each dx + 1 and dz + 1 of the
+// receiver's tile, 12 bits place in its slot (16 for arriving words).
+__device__ __forceinline__ void word_in(int2& e, int place, int reg) { e = make_int2(place, reg); }
+__device__ __forceinline__ void word_in(unsigned& e, int place, int reg) { e = (unsigned)place | (unsigned)reg << 16; }
+__device__ __forceinline__ void word_out(int2& e, int place, int reg, int dx, int dz, int llc, int llr) {
+  e = make_int2((dx + 1) * llc + (dz + 1) * llr + place, reg);
+}
+__device__ __forceinline__ void word_out(unsigned& e, int place, int reg, int dx, int dz, int, int) {
+  e = (unsigned)(place | (dz + 1) << 12 | (dx + 1) << 14) | (unsigned)reg << 16;
+}
+__device__ __forceinline__ int word_reg(int2 e) { return e.y; }
+__device__ __forceinline__ int word_reg(unsigned e) { return (int)(e >> 16); }
+__device__ __forceinline__ int word_from(int2 e) { return e.x; }
+__device__ __forceinline__ int word_from(unsigned e) { return (int)(e & 0xffff); }
+__device__ __forceinline__ int word_to(int2 e, int, int) { return e.x; }
+__device__ __forceinline__ int word_to(unsigned e, int llc, int llr) {
+  return (int)(e >> 14 & 3) * llc + (int)(e >> 12 & 3) * llr + (int)(e & 0xfff);
 }
 
 __device__ __forceinline__ void res_barrier(int threads) {
@@ -215,7 +243,7 @@ __device__ __forceinline__ void res_xline(const float (&u)[N + 1], const float (
 // nc: compute threads (the first of the CTA); the rest serve the receivers.  sw: lanes per tile
 // row (a power of two, at least the tile's columns of elements + 2: one for the left halo, one
 // for the nodes on the right); ezc: element rows per chunk.
-template <int N, int LPE, bool ADJ, bool STC>
+template <int N, int LPE, bool ADJ, bool STC, bool VG>
 __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
     sem_resident_kernel(const SolveDev* __restrict__ solves, const int* __restrict__ cta_solve,
                         const __grid_constant__ ResLay L, unsigned long long* __restrict__ ll,
@@ -224,6 +252,7 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
   constexpr int NP = N + 1, H2 = (N + 1) / 2;
   // two lanes per element (order 4): each has two columns' z-lines and two rows' x-lines and nodes
   static_assert(LPE == 1 || N == 4, "an element's halves");
+  static_assert(!VG || (ADJ && LPE == 1), "large adjoint tiles");
   constexpr int NJ = N / LPE, NQ = LPE == 2 ? 1 : H2;
   extern __shared__ __align__(128) float sm[];
   __shared__ SolveDev S;
@@ -286,6 +315,7 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
     for (int i = tid; i < Q.R * Q.C; i += T) {
       const int r = i / Q.C, cc = i - r * Q.C;
       const long long gi = (long long)(Q.gz0 + r) * S.pitch + Q.gx0 + cc;
+      if (VG) break;
       sm[L.v + r * L.Cp + cc] = vin[gi];
       if (ADJ) sm[L.g + r * L.Cp + cc] = S.grad[gi];
     }
@@ -295,40 +325,48 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
         sm[L.tz + 8 * i + 2 * q] = sm[L.tz + 8 * i + 2 * q + 1] = q < 2 ? f : -f;
       }
   }
-  // ---------------- exchange words that arrive: (place in this CTA's slot, region index)
-  int2* const win = reinterpret_cast<int2*>(sm + L.wi);
+  // ---------------- exchange words that arrive
+  typedef typename std::conditional<VG, unsigned, int2>::type Word;
+  Word* const win = reinterpret_cast<Word*>(sm + L.wi);
+  const int llc = kResSlots * L.llw, llr = llc * S.tiles_x;  // words of a tile, of a row of tiles
   const int nR = Q.R, nRN = Q.R * N, nC = Q.C, nCN = Q.C * N;
   const int n_in = (Q.hl ? nRN : 0) + (Q.ht ? nCN : 0) + (Q.hr ? nR : 0) + (Q.hb ? nC : 0) +
                    ((Q.hr && Q.hb && !ADJ) ? 1 : 0);
+  const int o0 = N * L.Wp + off + N;  // region index of the first owned node
   {
-    const int o0 = L.b + N * L.Wp + off + N;  // first owned node (of the first buffer)
     int n = 0;
-    if (Q.hl) { for (int w = tid; w < nRN; w += T) win[n + w] = make_int2(w, o0 + (w / N) * L.Wp - N + w % N); n += nRN; }
-    if (Q.ht) { for (int w = tid; w < nCN; w += T) win[n + w] = make_int2(L.ll_t + (w / nC) * L.Cm + w % nC, o0 + (w / nC - N) * L.Wp + w % nC); n += nCN; }
-    if (Q.hr) { for (int w = tid; w < nR; w += T) win[n + w] = make_int2(L.ll_r + w, o0 + w * L.Wp + Q.EX * N); n += nR; }
-    if (Q.hb) { for (int w = tid; w < nC; w += T) win[n + w] = make_int2(L.ll_b + w, o0 + nR * L.Wp + w); n += nC; }
-    if (Q.hr && Q.hb && !ADJ && tid == 0) win[n] = make_int2(L.ll_c, o0 + nR * L.Wp + Q.EX * N);
+    auto side = [&](bool has, int words, auto&& word) {
+      if (!has) return;
+      for (int w = tid; w < words; w += T) {
+        const int2 e = word(w);
+        word_in(win[n + w], e.x, e.y);
+      }
+      n += words;
+    };
+    side(Q.hl, nRN, [&](int w) { return make_int2(w, o0 + (w / N) * L.Wp - N + w % N); });
+    side(Q.ht, nCN, [&](int w) { return make_int2(L.ll_t + (w / nC) * L.Cm + w % nC, o0 + (w / nC - N) * L.Wp + w % nC); });
+    side(Q.hr, nR, [&](int w) { return make_int2(L.ll_r + w, o0 + w * L.Wp + Q.EX * N); });
+    side(Q.hb, nC, [&](int w) { return make_int2(L.ll_b + w, o0 + nR * L.Wp + w); });
+    side(Q.hr && Q.hb && !ADJ, 1, [&](int) { return make_int2(L.ll_c, o0 + nR * L.Wp + Q.EX * N); });
   }
-  // and words that leave, by the warp that advances the node: (region index, place in the
-  // receiver's slot 0); s_wo: each warp's range
-  int2* const wout = reinterpret_cast<int2*>(sm + L.wo);
+  // and words that leave, by the warp that advances the node; s_wo: each warp's range
+  Word* const wout = reinterpret_cast<Word*>(sm + L.wo);
   {
-    const int llc = kResSlots * L.llw, blk = blockIdx.x, o0 = L.b + N * L.Wp + off + N;
     const int n_r = Q.hr ? nRN : 0, n_b = Q.hb ? nCN : 0, n_l = Q.hl ? nR : 0, n_t = Q.ht ? nC : 0;
     const int n_out = n_r + n_b + n_l + n_t + ((Q.hl && Q.ht && !ADJ) ? 1 : 0);
     if (tid <= nw) s_wo[tid] = 0;
     __syncthreads();
     for (int pass = 0; pass < 2; ++pass) {
       for (int w = tid; w < n_out; w += T) {
-        int q = w, r, cc, to;
-        if (q < n_r) { r = q / N; cc = (Q.EX - 1) * N + q % N; to = (blk + 1) * llc + q; }
-        else if ((q -= n_r) < n_b) { r = nR - N + q / nC; cc = q % nC; to = (blk + S.tiles_x) * llc + L.ll_t + (q / nC) * L.Cm + cc; }
-        else if ((q -= n_b) < n_l) { r = q; cc = 0; to = (blk - 1) * llc + L.ll_r + q; }
-        else if ((q -= n_l) < n_t) { r = 0; cc = q; to = (blk - S.tiles_x) * llc + L.ll_b + q; }
-        else { r = 0; cc = 0; to = (blk - S.tiles_x - 1) * llc + L.ll_c; }
+        int q = w, r, cc, to, dx = 0, dz = 0;
+        if (q < n_r) { r = q / N; cc = (Q.EX - 1) * N + q % N; to = q; dx = 1; }
+        else if ((q -= n_r) < n_b) { r = nR - N + q / nC; cc = q % nC; to = L.ll_t + (q / nC) * L.Cm + cc; dz = 1; }
+        else if ((q -= n_b) < n_l) { r = q; cc = 0; to = L.ll_r + q; dx = -1; }
+        else if ((q -= n_l) < n_t) { r = 0; cc = q; to = L.ll_b + q; dz = -1; }
+        else { r = 0; cc = 0; to = L.ll_c; dx = dz = -1; }
         const int wp = (((r / N) / ezc) * sw + (cc / N + 1) * LPE + (r % N) / NJ) >> 5;
         const int at = atomicAdd(&s_wo[pass ? wp : wp + 1], 1);
-        if (pass) wout[at] = make_int2(o0 + r * L.Wp + cc, to);
+        if (pass) word_out(wout[at], to, o0 + r * L.Wp + cc, dx, dz, llc, llr);
       }
       __syncthreads();
       if (pass == 0 && tid == 0)
@@ -366,10 +404,12 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
   auto mis_tick = [&](int m) { return m >= S.it0 && m < S.it1 && (m - S.it0) % S.decim == 0; };
   auto y_at = [&](int m, int r) { return S.yobs[(long long)((m - S.it0) / S.decim) * S.nrec + r]; };
   int* const ioff = reinterpret_cast<int*>(sm + L.io);
-  int* const iterm = reinterpret_cast<int*>(sm + L.iq);
+  int* const s_iterm = reinterpret_cast<int*>(sm + L.iq);
   unsigned short* const imap = reinterpret_cast<unsigned short*>(sm + L.im);
   double ascale = 1.0;
   int niq = 0;               // injection: quads with receivers
+  const int* iterm = nullptr;  // their terms and weights (VG: in memory, which leaves room for a larger tile)
+  const float* iterm_w = nullptr;
   if (ADJ) {
     // the power of two that brings max|r| to ~1 (the tick kernels' scale tick)
     double m = 0.0;
@@ -388,8 +428,14 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
     for (int i = tid; i < niq; i += T) imap[(S.iq_pos[q0 + i] >> 16) * L.qx + (S.iq_pos[q0 + i] & 0xffff)] = i + 1;
     for (int i = tid; i <= niq; i += T) ioff[i] = S.iterm_off[q0 + i] - e0;
     const int ne = S.iterm_off[q0 + niq] - e0;
-    for (int i = tid; i < ne; i += T) iterm[i] = S.iterm[e0 + i];
-    for (int i = tid; i < ne * N; i += T) sm[L.ie + i] = S.iterm_w[(long long)e0 * N + i];
+    iterm = S.iterm + e0;
+    iterm_w = S.iterm_w + (long long)e0 * N;
+    if (!VG) {
+      for (int i = tid; i < ne; i += T) s_iterm[i] = iterm[i];
+      for (int i = tid; i < ne * N; i += T) sm[L.ie + i] = iterm_w[i];
+      iterm = s_iterm;
+      iterm_w = sm + L.ie;
+    }
   }
   auto residual = [&](int t) -> float {  // the adjoint source term of this thread's receiver at step t
     if (!mis_tick(t)) return 0.f;
@@ -410,7 +456,7 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
           const float r = rs[e >> 8];
 #pragma unroll
           for (int i = 0; i < N; ++i)
-            if ((e >> i) & 1) acc[i] = __fmaf_rn(sm[L.ie + k * N + i], r, acc[i]);
+            if ((e >> i) & 1) acc[i] = __fmaf_rn(iterm_w[k * N + i], r, acc[i]);
         }
 #pragma unroll
       for (int i = 0; i < N; ++i) sm[L.ia + (t & 1) * (L.niq * N) + q * N + i] = acc[i];
@@ -464,15 +510,16 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
   const bool fin = !ADJ && kind == RES_FWD && shift;  // one more read-out after the last step
   const int nst = t_hi - t_lo;                        // steps
   int n_fail = -1;
-  const unsigned long long* const in0 = ll + (long long)blockIdx.x * kResSlots * L.llw;
+  const unsigned long long* const in0 = ll + (long long)blockIdx.x * llc;
+  unsigned long long* const ll_out = ll + ((long long)blockIdx.x * llc - llc - llr);  // the tile above on the left
   // wait for the edge words of step n's field and put them into the halo (every thread takes part)
   auto receive = [&](const int n) {
     const unsigned tag = tag0 + (unsigned)n;
     const int so = (int)(tag & (kResSlots - 1)) * L.llw;
-    float* const f = sm + (n & 1) * L.reg;
+    float* const f = sm + L.b + (n & 1) * L.reg;
 #pragma unroll 1
     for (int w0 = tid; w0 < n_in; w0 += 4 * T) {  // up to four words of a thread in flight
-      int2 e[4];
+      Word e[4];
       unsigned long long v[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) e[j] = win[w0 + j * T < n_in ? w0 + j * T : w0];
@@ -482,7 +529,7 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
         bool ok = true;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (j == 0 || w0 + j * T < n_in) v[j] = ll_load(in0 + so + e[j].x);
+          if (j == 0 || w0 + j * T < n_in) v[j] = ll_load(in0 + so + word_from(e[j]));
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           if (j == 0 || w0 + j * T < n_in) ok &= (unsigned)(v[j] >> 32) == tag;
@@ -495,7 +542,7 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        if (j == 0 || w0 + j * T < n_in) f[e[j].y] = __uint_as_float((unsigned)v[j]);
+        if (j == 0 || w0 + j * T < n_in) f[word_reg(e[j])] = __uint_as_float((unsigned)v[j]);
     }
   };
   // ---------------- receiver threads' state
@@ -706,6 +753,42 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
       const int ri = oc + r0 * L.Wp, oi = r0 * L.Cp + ec * N;
       float2 X[NJ][H2], SX[NJ][H2];
       float re[NJ], rs[NJ];
+      const bool mine = owner && on;
+      float2 v[NJ][H2], g[NJ][H2];
+      // a row of the increment or the partial gradient: in shared memory, or (VG) in the solve's fields
+      auto vg_at = [&](int j, int o, float* f) { return VG ? f + (Q.gz0 + r0 + j) * pitch + Q.gx0 + ec * N : sm + o + oi + j * L.Cp; };
+      auto vg_get = [&](float2 (&x)[NJ][H2], int o, float* f) {
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const float* const p = vg_at(j, o, f);
+          if constexpr (!VG || N == 4) {
+            if (!VG || (mine && (j == 0 || !vz))) get2<N>(p, x[j]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+              const float a = mine && (j == 0 || !vz) && (full || i == 0) ? p[i] : 0.f;
+              if (i & 1) x[j][i / 2].y = a; else x[j][i / 2].x = a;
+            }
+          }
+        }
+      };
+      auto vg_put = [&](float2 (&x)[NJ][H2], int o, float* f) {
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          float* const p = vg_at(j, o, f);
+          if constexpr (!VG || N == 4) {
+            if (!VG || j == 0 || !vz) put2<N>(p, x[j]);
+          } else if (j == 0 || !vz) {
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+              if (full || i == 0) p[i] = lane_of(x[j], i);
+          }
+        }
+      };
+      if constexpr (VG) {  // (in flight during the x-lines)
+        vg_get(v, L.v, S.Mu);
+        vg_get(g, L.g, S.grad);
+      }
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
         float lu[NP], lc[NP], lw[NP];
@@ -726,7 +809,6 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
         }
       }
       // (nodes past the mesh's last line or column lie in this tile's arrays too and stay 0)
-      const bool mine = owner && on;
       float4 tz[NJ];   // 1/m_z and R_z, twice each
       float2 ndz[NJ];
 #pragma unroll
@@ -735,9 +817,7 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
         ndz[j] = *reinterpret_cast<const float2*>(sm + L.tz + 8 * (r0 + j) + 4);
       }
       if constexpr (ADJ) {
-        float2 g[NJ][H2];
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) get2<N>(sm + L.g + oi + j * L.Cp, g[j]);
+        if constexpr (!VG) vg_get(g, L.g, nullptr);
 #pragma unroll
         for (int j = 0; j < NJ; ++j)
 #pragma unroll
@@ -760,14 +840,9 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
         for (int j = 0; j < NJ; ++j)
 #pragma unroll
           for (int i = 0; i < H2; ++i) g[j][i] = __fadd2_rn(g_start ? make_float2(0.f, 0.f) : g[j][i], SX[j][i]);
-        if (mine) {
-#pragma unroll
-          for (int j = 0; j < NJ; ++j) put2<N>(sm + L.g + oi + j * L.Cp, g[j]);
-        }
+        if (mine) vg_put(g, L.g, S.grad);
       }
-      float2 v[NJ][H2];
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) get2<N>(sm + L.v + oi + j * L.Cp, v[j]);
+      if constexpr (!VG) vg_get(v, L.v, nullptr);
       if constexpr (STC) {
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
@@ -853,10 +928,8 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
       }
       if (mine) {
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-          put2<N>(fn + ri + j * L.Wp, X[j]);
-          put2<N>(sm + L.v + oi + j * L.Cp, v[j]);
-        }
+        for (int j = 0; j < NJ; ++j) put2<N>(fn + ri + j * L.Wp, X[j]);
+        vg_put(v, L.v, S.Mu);
         if (!ADJ && bo) {
           float* const p = bo + (Q.gz0 + r0) * pitch + Q.gx0 + ec * N;
 #pragma unroll
@@ -877,18 +950,19 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
     if (more || fin) {
       __syncwarp();
       const unsigned tag = tag0 + (unsigned)n + 1;
-      unsigned long long* const p = ll + (int)(tag & (kResSlots - 1)) * L.llw;
-      const float* const f = sm + ((n + 1) & 1) * L.reg;
+      unsigned long long* const p = ll_out + (int)(tag & (kResSlots - 1)) * L.llw;
+      const float* const f = sm + L.b + ((n + 1) & 1) * L.reg;
 #pragma unroll 1
       for (int w0 = w_lo + lane; w0 < w_hi; w0 += 128) {
-        int2 e[4];
+        Word e[4];
         float v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) e[j] = wout[min(w0 + 32 * j, w_hi - 1)];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = f[e[j].x];
+        for (int j = 0; j < 4; ++j) v[j] = f[word_reg(e[j])];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) ll_send(p + e[j].y, v[j], tag);  // (past the end: the last word again)
+        for (int j = 0; j < 4; ++j)  // (past the end: the last word again)
+          ll_send(p + word_to(e[j], llc, llr), v[j], tag);
       }
     }
     // ---- now and then: v at a checkpoint, the gradient's partial sums into the float64 field (while
@@ -908,7 +982,7 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
           for (int i = 0; i < N; ++i) a[i] = (full || i == 0) ? S.grad64[gi + i] : 0.0;
 #pragma unroll
           for (int i = 0; i < N; ++i)
-            if (full || i == 0) S.grad64[gi + i] = __dadd_rn(a[i], (double)sm[L.g + oi + i]);
+            if (full || i == 0) S.grad64[gi + i] = __dadd_rn(a[i], (double)(VG ? S.grad[gi + i] : sm[L.g + oi + i]));
         }
       }
     }
@@ -935,6 +1009,7 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
     if (more) {
       const long long gi = (long long)(Q.gz0 + r) * S.pitch + Q.gx0 + cc;
       S.L[(long long)(t_lo & 1) * S.fstride + gi] = f;
+      if (VG) continue;
       S.Mu[gi] = sm[L.v + r * L.Cp + cc];
       S.grad[gi] = sm[L.g + r * L.Cp + cc];
     }

@@ -7,24 +7,41 @@ SolveIo solve_io(const sem_solve_t& s, const Workspace& ws, char* a);
 
 typedef void (*ResFn)(const SolveDev*, const int*, ResLay, unsigned long long*, unsigned, int, int, int, int, int);
 
+// variants: one lane per element, two (order 4), one with the increment and the partial gradient in
+// memory (adjoint, for meshes whose tiles fit in no other way: 400x200 alone, forward + adjoint, 15.7 us
+// a step, 27.7 by strips; not above order 4, where its registers spill: order 5, 240x150, 26.0 us, 24.2
+// by strips)
+enum : int { RES_ONE = 1, RES_TWO = 2, RES_MEM = 3 };
+int res_lanes(int vr) { return vr == RES_TWO ? 2 : 1; }
+bool res_has(int N, int vr, bool adj) { return vr == RES_ONE || (vr == RES_TWO && N == 4) || (vr == RES_MEM && adj && N <= 4); }
+
+template <int N, bool ADJ, bool STC>
+ResFn res_fn(int vr) {
+  if constexpr (N == 4) {
+    if (vr == RES_TWO) return sem_resident_kernel<N, 2, ADJ, STC, false>;
+  }
+  if constexpr (ADJ && N <= 4) {
+    if (vr == RES_MEM) return sem_resident_kernel<N, 1, ADJ, STC, true>;
+  }
+  return sem_resident_kernel<N, 1, ADJ, STC, false>;
+}
 template <bool ADJ, bool STC>
-ResFn res_fn(int N, int lpe) {
+ResFn res_fn(int N, int vr) {
   switch (N) {
-    case 1: return sem_resident_kernel<1, 1, ADJ, STC>;
-    case 2: return sem_resident_kernel<2, 1, ADJ, STC>;
-    case 3: return sem_resident_kernel<3, 1, ADJ, STC>;
-    case 4: return lpe == 2 ? sem_resident_kernel<4, 2, ADJ, STC> : sem_resident_kernel<4, 1, ADJ, STC>;
-    case 5: return sem_resident_kernel<5, 1, ADJ, STC>;
-    case 6: return sem_resident_kernel<6, 1, ADJ, STC>;
-    case 7: return sem_resident_kernel<7, 1, ADJ, STC>;
+    case 1: return res_fn<1, ADJ, STC>(vr);
+    case 2: return res_fn<2, ADJ, STC>(vr);
+    case 3: return res_fn<3, ADJ, STC>(vr);
+    case 4: return res_fn<4, ADJ, STC>(vr);
+    case 5: return res_fn<5, ADJ, STC>(vr);
+    case 6: return res_fn<6, ADJ, STC>(vr);
+    case 7: return res_fn<7, ADJ, STC>(vr);
   }
   return nullptr;
 }
-ResFn res_kernel_for(int N, int lpe, bool adj, bool stc) {
-  if (adj) return stc ? res_fn<true, true>(N, lpe) : res_fn<true, false>(N, lpe);
-  return stc ? res_fn<false, true>(N, lpe) : res_fn<false, false>(N, lpe);
+ResFn res_kernel_for(int N, int vr, bool adj, bool stc) {
+  if (adj) return stc ? res_fn<true, true>(N, vr) : res_fn<true, false>(N, vr);
+  return stc ? res_fn<false, true>(N, vr) : res_fn<false, false>(N, vr);
 }
-int res_max_lanes(int N) { return N == 4 ? 2 : 1; }  // lanes per element
 
 // Receiver lists of the balanced tiling ntx x ntz of a plan (tiles from res_start).
 int get_res_lists(const sem_plan_s* p, int ntx, int ntz, sem_plan_s::ResLists* out) {
@@ -101,17 +118,17 @@ void take_max(ResCounts& a, const ResCounts& b) {
   a.nquad = std::max(a.nquad, b.nquad); a.nterm = std::max(a.nterm, b.nterm);
 }
 
-ResLay res_layout(int N, int lpe, bool adj, bool stc, int exm, int ezm, const ResCounts& c) {
+ResLay res_layout(int N, int vr, bool adj, bool stc, int exm, int ezm, int ezl, const ResCounts& c) {
   ResLay L{};
   const int NP = N + 1;
   // rows of lanes spread over the banks: two lanes per element read rows two apart at once
-  auto pitch = [&](int v) { return lpe == 2 ? (v + 7) / 16 * 16 + 8 : 4 * ((v + 3) / 4 | 1); };
+  auto pitch = [&](int v) { return vr == RES_TWO ? (v + 7) / 16 * 16 + 8 : 4 * ((v + 3) / 4 | 1); };
   L.Rm = ezm * N + 1;
   L.Cm = exm * N + 1;
   L.qx = exm + 1;
   L.Wp = pitch((N == 4 ? 0 : 4) + N + (exm + 1) * N);
   L.Cp = pitch((exm + 1) * N);
-  const int rows = (ezm + 1) * N;  // one more element row: the mesh's last line of nodes starts it
+  const int rows = std::max(ezm, ezl + 1) * N;  // in the last tiles the mesh's last line of nodes starts an element row
   L.H = N + rows + 1;
   int o = 0;
   auto take = [&](long long n, int align = 4) { o = (int)round_up(o, align); const int at = o; o += (int)n; return at; };
@@ -119,19 +136,22 @@ ResLay res_layout(int N, int lpe, bool adj, bool stc, int exm, int ezm, const Re
   L.wreg = (int)round_up(L.reg, 32);
   const int own = L.Cp * rows;
   if (adj) L.w = take(2LL * L.wreg, 32);
-  L.b = take(2LL * L.reg); L.c = take(L.reg); L.v = take(own);
-  if (adj) L.g = take(own);
+  L.b = take(2LL * L.reg); L.c = take(L.reg);
+  if (vr != RES_MEM) L.v = take(own);
+  if (adj && vr != RES_MEM) L.g = take(own);
   L.tz = take(8LL * rows);
   const long long words = (long long)(L.Rm + L.Cm) * NP + 1;
-  L.wi = take(2 * words); L.wo = take(2 * words);
+  L.wi = take(vr == RES_MEM ? words : 2 * words); L.wo = take(vr == RES_MEM ? words : 2 * words);
   if (adj) {
     L.nrm = std::max(1, c.ninj);
     L.niq = c.nquad;
     L.rs = take(4LL * L.nrm);
     L.ia = take(2LL * c.nquad * N);
     L.io = take((long long)c.nquad + 1);
-    L.iq = take(c.nterm);
-    L.ie = take((long long)c.nterm * N);
+    if (vr != RES_MEM) {
+      L.iq = take(c.nterm);
+      L.ie = take((long long)c.nterm * N);
+    }
     L.im = take(((long long)rows * L.qx + 1) / 2);
   }
   if (stc) { const int bn = 2 * L.Rm + L.Cm; L.be = take(3LL * bn); L.bd = take(2LL * bn); }
@@ -141,17 +161,17 @@ ResLay res_layout(int N, int lpe, bool adj, bool stc, int exm, int ezm, const Re
   return L;
 }
 
-constexpr int kResSmem = 230400;  // dynamic shared bytes: one CTA per SM
+constexpr int kResSmem = 231424;  // dynamic shared bytes: one CTA per SM, 1 KB left for its static ones
 // Threads of a launch whose largest tile is exm x ezm elements (the lowest ezl high): lanes per
 // tile row, element rows per chunk, compute and receiver threads; exchange words.
 struct ResShape { int sw, ezc, nc, nio, edge; };
-bool res_shape(int N, int lpe, bool adj, int exm, int ezm, int ezl, int nrec, ResShape* h) {
+bool res_shape(int N, int vr, bool adj, int exm, int ezm, int ezl, int nrec, ResShape* h) {
   const int ezr = std::max(ezm, ezl + 1);  // element rows, the mesh's last line of nodes counted as one
   h->nio = (int)round_up(std::max(nrec, 1), 32);
   h->edge = (exm + ezm) * N * (N + 1);
-  const int tmax = res_threads(lpe, adj) - h->nio;
+  const int tmax = res_threads(res_lanes(vr), adj) - h->nio;
   h->sw = 4;
-  while (h->sw < (exm + 2) * lpe) h->sw *= 2;
+  while (h->sw < (exm + 2) * res_lanes(vr)) h->sw *= 2;
   if (h->sw > 32 || tmax < 32) return false;
   h->ezc = (ezr + tmax / h->sw - 1) / (tmax / h->sw);
   h->nc = (int)round_up((long long)((ezr + h->ezc - 1) / h->ezc) * h->sw, 32);
@@ -166,20 +186,23 @@ bool res_shape(int N, int lpe, bool adj, int exm, int ezm, int ezl, int nrec, Re
 // swaps between them, which decides full SMs (128 of 100x50: 133 us a step, 142 with two).
 // Two or three smaller CTAs per SM, which hide one another's exchange, measured the same or
 // slower (16 of 100x50 with one lane: 18.1 us a step with one, 18.9 with two, 22.5 with three).
-double res_step_cost(int N, int lpe, bool adj, const ResShape& h) {
+double res_step_cost(int N, int vr, bool adj, const ResShape& h) {
   const double NP = N + 1;
   const double el = adj ? 2 * N * (3 * NP * NP + 4 * NP) + 16 * N * N : 2 * N * (2 * NP * NP + 2 * NP) + 10 * N * N;
   const double carry = N * (NP * NP + 3 * NP) + (adj ? N * (NP + 2) : 0);
-  const double fixed = lpe == 2 ? 2600.0 : adj ? 2300.0 : 2500.0, rate = !adj ? 1.6 : lpe == 2 ? 1.7 : 1.9;
-  return fixed + 1.2 * h.edge + rate * std::max(1.0, h.nc / 128.0) * (h.ezc * el + carry) / lpe;
+  const double fixed = vr == RES_TWO ? 2600.0 : adj ? 2300.0 : 2500.0;
+  const double rate = !adj ? 1.6 : vr == RES_TWO ? 1.7 : vr == RES_ONE ? 1.9 : 2.1;
+  return fixed + 1.2 * h.edge + rate * std::max(1.0, h.nc / 128.0) * (h.ezc * el + carry) / res_lanes(vr);
 }
-bool res_fits(const ResLay& L) { return L.Wp <= 256 && L.H <= 256 && (long long)L.total * 4 <= kResSmem; }
+bool res_fits(const ResLay& L) {  // (256: the history box; 4096: the place of a packed exchange word)
+  return L.Wp <= 256 && L.H <= 256 && L.llw <= 4096 && (long long)L.total * 4 <= kResSmem;
+}
 
 // bounds of the receivers of one tile of a tiling
 ResCounts res_counts(const sem_plan_s* p, int ntx, int ntz) {
   ResCounts c;
   const int N = p->npol;
-  std::map<int, std::pair<int, std::vector<int>>> tiles;  // receivers and their elements
+  std::map<int, std::pair<int, std::vector<int>>> tiles;  // receivers and the quads of their first rows
   for (int r = 0; r < p->nrec; ++r) {
     const int ex = p->h_rec_base[2 * r] / N, ez = p->h_rec_base[2 * r + 1] / N;
     int seen[4], ns = 0;
@@ -192,24 +215,26 @@ ResCounts res_counts(const sem_plan_s* p, int ntx, int ntz) {
       seen[ns++] = t;
       auto& e = tiles[t];
       e.first++;
-      if (std::find(e.second.begin(), e.second.end(), ez * p->nelx + ex) == e.second.end())
-        e.second.push_back(ez * p->nelx + ex);
+      for (int i = 0; i < 2; ++i) {
+        const int quad = ez * (p->nelx + 1) + ex + i;
+        if (std::find(e.second.begin(), e.second.end(), quad) == e.second.end()) e.second.push_back(quad);
+      }
     }
   }
   for (auto& kv : tiles) {
     c.nrec = std::max(c.nrec, kv.second.first);
-    c.nquad = std::max(c.nquad, (int)kv.second.second.size() * 2 * (N + 1));
+    c.nquad = std::max(c.nquad, (int)kv.second.second.size() * (N + 1));
   }
   c.ninj = c.nrec;
   c.nterm = c.ninj * 2 * (N + 1);
   return c;
 }
 
-// Tiling of a plan into tiles of at most E elements that fit a CTA: the one with the least work
-// (tiles times modelled step); kept with the plan.  0 x 0: none.
-ResTiling res_tiling(const sem_plan_s* p, int lpe, bool adj, int E) {
+// Tiling of a plan into at most sms tiles of at most E elements that fit a CTA: the one with the
+// least work (tiles times modelled step); kept with the plan.  0 x 0: none.
+ResTiling res_tiling(const sem_plan_s* p, int vr, bool adj, int E, int sms) {
   std::lock_guard<std::mutex> lk(p->mu);
-  const auto key = std::make_tuple(lpe, adj, E);
+  const auto key = std::make_tuple(vr, adj, E);
   auto it = p->res_tilings.find(key);
   if (it != p->res_tilings.end()) return it->second;
   ResTiling best;
@@ -219,15 +244,16 @@ ResTiling res_tiling(const sem_plan_s* p, int lpe, bool adj, int E) {
     const int ex = (p->nelx + tx - 1) / tx;
     if (tx > 1 && ex == (p->nelx + tx - 2) / (tx - 1)) continue;  // no narrower than with one tile less
     const int ezm = E / ex;
-    if (ezm < 1 || (ex + 2) * lpe > 32) continue;
+    if (ezm < 1 || (ex + 2) * res_lanes(vr) > 32) continue;
     const int tz = (p->nelz + ezm - 1) / ezm, ez = (p->nelz + tz - 1) / tz;
+    if ((long long)tx * tz > sms) continue;
     ResShape h;
-    if (!res_shape(p->npol, lpe, adj, ex, ez, p->nelz / tz, 1, &h)) continue;
-    const double c = res_step_cost(p->npol, lpe, adj, h);
+    if (!res_shape(p->npol, vr, adj, ex, ez, p->nelz / tz, 1, &h)) continue;
+    const double c = res_step_cost(p->npol, vr, adj, h);
     if (best_c >= 0.0 && tx * tz * c >= best_c) continue;
     const ResCounts cnt = res_counts(p, tx, tz);
-    if (!res_shape(p->npol, lpe, adj, ex, ez, p->nelz / tz, adj ? cnt.ninj : cnt.nrec, &h) ||
-        !res_fits(res_layout(p->npol, lpe, adj, stc, ex, ez, cnt)))
+    if (!res_shape(p->npol, vr, adj, ex, ez, p->nelz / tz, adj ? cnt.ninj : cnt.nrec, &h) ||
+        !res_fits(res_layout(p->npol, vr, adj, stc, ex, ez, p->nelz / tz, cnt)))
       continue;
     best.tx = tx; best.tz = tz;
     best.n = cnt;
@@ -237,10 +263,33 @@ ResTiling res_tiling(const sem_plan_s* p, int lpe, bool adj, int E) {
   return best;
 }
 
+// Tile capacities that are tried: 8 to 1200 elements
+template <class F>
+void res_capacities(F&& f) {
+  for (double E = 8.0; E < 1200.0; E *= 1.15) f((int)E);
+}
+// The variants a plan's solve needs by itself: RES_ONE (or RES_TWO), RES_MEM (its adjoint tiles fit
+// in no other way) or 0 (too large).
+int res_need(const sem_plan_s* p, bool adj, int sms) {
+  {
+    std::lock_guard<std::mutex> lk(p->mu);
+    if (p->res_need[adj] >= 0) return p->res_need[adj];
+  }
+  auto any = [&](int vr, bool a) {
+    bool fit = false;
+    if (res_has(p->npol, vr, a)) res_capacities([&](int E) { fit = fit || res_tiling(p, vr, a, E, sms).tx > 0; });
+    return fit;
+  };
+  int need = any(RES_ONE, false) || any(RES_TWO, false) ? RES_ONE : 0;
+  if (need && adj) need = any(RES_ONE, true) || any(RES_TWO, true) ? RES_ONE : any(RES_MEM, true) ? RES_MEM : 0;
+  std::lock_guard<std::mutex> lk(p->mu);
+  return p->res_need[adj] = need;
+}
+
 // Waves of one kernel over a group of solves: each solve's tiling, and the solves (places in the
 // group) whose CTAs are resident at once.  A wave's launch shape is its largest tile's.
 struct ResPack {
-  int lpe = 0;
+  int vr = 0;          // variant
   double cost = -1.0;  // modelled cycles; < 0: a solve does not fit
   std::vector<ResTiling> tiles;
   std::vector<std::vector<int>> waves;
@@ -265,16 +314,17 @@ ResPack res_pack(const sem_solve_t* sv, const std::vector<int>& idx, const std::
   ResPack best;
   std::vector<ResTiling> tl(plans.size()), last;
   std::vector<int> first;
-  for (int lpe = 1; lpe <= res_max_lanes(N); ++lpe) {
+  for (int vr = RES_ONE; vr <= RES_MEM; ++vr) {
+    if (!res_has(N, vr, adj)) continue;
     last.clear();
-    for (double Ed = 8.0; Ed < 1200.0; Ed *= 1.15) {
+    res_capacities([&](int E) {
       bool ok = true, same = !last.empty();
       for (size_t q = 0; q < plans.size() && ok; ++q) {
-        tl[q] = res_tiling(plans[q], lpe, adj, (int)Ed);
-        ok = tl[q].tx > 0 && (long long)tl[q].tx * tl[q].tz <= sms;
+        tl[q] = res_tiling(plans[q], vr, adj, E, sms);
+        ok = tl[q].tx > 0;
         same = same && tl[q].tx == last[q].tx && tl[q].tz == last[q].tz;
       }
-      if (!ok || same) continue;
+      if (!ok || same) return;
       last = tl;
       first.clear();
       double cost = 0.0, step = 0.0;
@@ -290,26 +340,26 @@ ResPack res_pack(const sem_solve_t* sv, const std::vector<int>& idx, const std::
         bool fits = j > 0 && used + t.tx * t.tz <= sms;
         if (fits) {
           const int x = std::max(ex, exm), z = std::max(ez, ezm);
-          fits = res_shape(N, lpe, adj, x, z, std::max(el, ezl), adj ? c.ninj : c.nrec, &h) &&
-                 res_fits(res_layout(N, lpe, adj, stc, x, z, c));
+          fits = res_shape(N, vr, adj, x, z, std::max(el, ezl), adj ? c.ninj : c.nrec, &h) &&
+                 res_fits(res_layout(N, vr, adj, stc, x, z, std::max(el, ezl), c));
         }
         if (!fits) {  // the next wave
           cost += step * nt;
           first.push_back(j);
           used = nt = exm = ezm = ezl = 0;
           c = t.n;
-          res_shape(N, lpe, adj, ex, ez, el, adj ? c.ninj : c.nrec, &h);
+          res_shape(N, vr, adj, ex, ez, el, adj ? c.ninj : c.nrec, &h);
         }
         cnt = c;
         used += t.tx * t.tz;
         exm = std::max(exm, ex); ezm = std::max(ezm, ez); ezl = std::max(ezl, el);
-        step = res_step_cost(N, lpe, adj, h);
+        step = res_step_cost(N, vr, adj, h);
         nt = std::max(nt, steps[j]);
       }
       cost += step * nt;
-      if (best.cost >= 0.0 && cost >= best.cost) continue;
+      if (best.cost >= 0.0 && cost >= best.cost) return;
       best.cost = cost;
-      best.lpe = lpe;
+      best.vr = vr;
       best.tiles.resize(n);
       for (int j = 0; j < n; ++j) best.tiles[j] = tl[pl[j]];
       best.waves.clear();
@@ -317,7 +367,7 @@ ResPack res_pack(const sem_solve_t* sv, const std::vector<int>& idx, const std::
         best.waves.emplace_back();
         for (int j = first[w]; j < (w + 1 < first.size() ? first[w + 1] : n); ++j) best.waves.back().push_back(j);
       }
-    }
+    });
   }
   return best;
 }
@@ -420,9 +470,9 @@ int run_res_group(sem_batch_t* b, const sem_solve_t* sv, const ResGroup& w, int 
       v.cta0 = cta0;
       cta0 += v.ncta;
       v.solves = &wv;
-      v.L = res_layout(N, pk.lpe, q, stc, exm, ezm, c);
-      v.fn = res_kernel_for(N, pk.lpe, q, stc);
-      if (!res_shape(N, pk.lpe, q, exm, ezm, ezl, q ? c.ninj : c.nrec, &v.h)) return SEM_ERR_UNSUPPORTED;
+      v.L = res_layout(N, pk.vr, q, stc, exm, ezm, ezl, c);
+      v.fn = res_kernel_for(N, pk.vr, q, stc);
+      if (!res_shape(N, pk.vr, q, exm, ezm, ezl, q ? c.ninj : c.nrec, &v.h)) return SEM_ERR_UNSUPPORTED;
       int nb = 0;
       if (!res_fits(v.L) || raise_smem_limit((const void*)v.fn, (size_t)v.L.total * 4) != cudaSuccess ||
           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, v.fn, v.h.nc + v.h.nio, (size_t)v.L.total * 4) != cudaSuccess ||
@@ -640,9 +690,16 @@ int run_resident(sem_batch_t* b, const sem_solve_t* sv, int n, long long budget,
                  std::vector<int>* rest) {
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-  std::map<std::tuple<int, bool, bool>, std::vector<int>> classes;
-  for (int i = 0; i < n; ++i)
-    classes[std::make_tuple(sv[i].plan->npol, sv[i].plan->bnd_n > 0, (sv[i].flags & SEM_F_ADJOINT) != 0)].push_back(i);
+  std::map<std::tuple<int, bool, bool, int>, std::vector<int>> classes;
+  for (int i = 0; i < n; ++i) {
+    const sem_plan_s* p = sv[i].plan;
+    const bool adj = sv[i].flags & SEM_F_ADJOINT;
+    const int need = res_need(p, adj, sms);
+    // adjoint solves too large for shared memory that were given a checkpoint interval keep the strip
+    // kernel, whose schedule the interval was chosen for
+    if (!need || (need == RES_MEM && sv[i].ckpt_k > 0 && sv[i].ckpt_k < p->nt)) rest->push_back(i);
+    else classes[std::make_tuple(p->npol, p->bnd_n > 0, adj, need)].push_back(i);
+  }
   for (auto& kv : classes) {
     const std::vector<ResGroup> groups = res_plan(sv, kv.second, sms, budget);
     if (groups.empty()) { rest->insert(rest->end(), kv.second.begin(), kv.second.end()); continue; }

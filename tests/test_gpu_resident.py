@@ -117,3 +117,12 @@ def test_non_finite_velocity_is_reported():
     s.velocity[17] = float("inf")
     Batch(kernel=5).run([s])
     assert int(s.status.item()) != 0
+
+
+@pytest.mark.parametrize("npol,nelx,nelz,boundary", [
+    (3, 420, 270, "sponge"), (4, 330, 171, "sponge"), (4, 345, 180, "stacey")])
+def test_adjoint_tiles_with_fields_in_memory(npol, nelx, nelz, boundary):
+    # meshes whose adjoint tiles only fit with the increment and the partial gradient in memory
+    p, c = _plan(nelx, nelz, npol, 120, 8, boundary, circle=True)
+    b = _compare(lambda: [_spec(p, c, 3, "gradient")])
+    assert b.last_kernel == "resident"

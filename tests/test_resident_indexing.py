@@ -11,11 +11,11 @@ def pitch(lpe, v):
 class Layout:
     """The fields of ResLay that index arithmetic uses."""
 
-    def __init__(self, N, lpe, exm, ezm):
+    def __init__(self, N, lpe, exm, ezm, ezl):
         self.N, self.Rm, self.Cm, self.qx = N, ezm * N + 1, exm * N + 1, exm + 1
         self.Wp = pitch(lpe, (0 if N == 4 else 4) + N + (exm + 1) * N)
         self.Cp = pitch(lpe, (exm + 1) * N)
-        self.rows = (ezm + 1) * N
+        self.rows = max(ezm, ezl + 1) * N
         self.H = N + self.rows + 1
         self.t = self.Rm * N
         self.r = self.t + self.Cm * N
@@ -80,7 +80,7 @@ def sends(T, L, t, ntx):
     (4, 8, 8, 1, 5, 1), (4, 8, 8, 1, 5, 2), (5, 7, 9, 3, 2, 1), (6, 5, 5, 2, 3, 1), (7, 4, 4, 3, 2, 1)])
 def test_exchange_and_bounds(N, nelx, nelz, ntx, ntz, lpe):
     exm, ezm = -(-nelx // ntx), -(-nelz // ntz)
-    L = Layout(N, lpe, exm, ezm)
+    L = Layout(N, lpe, exm, ezm, nelz // ntz)
     tiles = [Tile(N, nelx, nelz, ntx, ntz, t) for t in range(ntx * ntz)]
     assert sum(T.R * T.C for T in tiles) == (nelx * N + 1) * (nelz * N + 1)
     sent = {}
@@ -89,6 +89,10 @@ def test_exchange_and_bounds(N, nelx, nelz, ntx, ntz, lpe):
         for to, word, r, c in sends(T, L, t, ntx):
             assert 0 <= to < len(tiles) and 0 <= word < L.words
             assert (to, word) not in sent
+            # a packed word's fields: place, offset of the receiver's tile, region index
+            dx, dz = to % ntx - t % ntx, to // ntx - t // ntx
+            assert word < 4096 and abs(dx) <= 1 and abs(dz) <= 1 and to == t + dx + dz * ntx
+            assert (N + r) * L.Wp + T.off + N + c < min(65536, L.Wp * L.H)
             sent[to, word] = (T.gx0 + c, T.gz0 + r)
     wanted = set()
     for t, T in enumerate(tiles):
