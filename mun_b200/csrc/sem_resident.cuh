@@ -40,9 +40,9 @@
 // Arithmetic.  Per node the operations and roundings of the tile and strip kernels, in the
 // same order: results are bitwise equal to theirs.
 
-// most threads of a resident CTA, by lanes per element: 168 (forward) and 255 (adjoint) registers
-// each with one, 128 with two
-__host__ __device__ constexpr int res_threads(int lpe, bool adj) { return lpe == 2 ? 512 : adj ? 256 : 384; }
+// most threads of a resident CTA, by order, lanes per element and kernel: up to 255 registers each
+// with 256, 168 with 384, 128 with 512
+__host__ __device__ constexpr int res_threads(int N, int lpe, bool adj) { return lpe == 2 ? 512 : adj || N > 4 ? 256 : 384; }
 constexpr int kResSlots = 4;       // exchange slots by step tag
 
 // Shared-memory layout (float offsets) and exchange layout (words) of one launch, by its
@@ -244,7 +244,7 @@ __device__ __forceinline__ void res_xline(const float (&u)[N + 1], const float (
 // row (a power of two, at least the tile's columns of elements + 2: one for the left halo, one
 // for the nodes on the right); ezc: element rows per chunk.
 template <int N, int LPE, bool ADJ, bool STC, bool VG>
-__global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
+__global__ void __launch_bounds__(res_threads(N, LPE, ADJ), 1)
     sem_resident_kernel(const SolveDev* __restrict__ solves, const int* __restrict__ cta_solve,
                         const __grid_constant__ ResLay L, unsigned long long* __restrict__ ll,
                         const unsigned tag0, const int kind, const int idx, const int nc, const int sw,
@@ -590,11 +590,8 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
   }
   const int src_i = (S.src_gx - Q.gx0) % N;
   const int pitch = S.pitch;
-  // Stacey: local slot of an absorbing-edge node of this tile, or -1
-  auto edge_of = [&](int r, int c) -> int {
-    if (Q.gz0 + r == 0 || r >= Q.R || c >= Q.C) return -1;
-    return (!Q.hl && c == 0) ? r : (!Q.hr && c == Q.C - 1) ? L.Rm + r : (!Q.hb && r == Q.R - 1) ? 2 * L.Rm + c : -1;
-  };
+  // Stacey: local slot of this lane's first node of row 0 on an absorbing side, or -1
+  const int side = !stc_edge ? -1 : (el == 1 && !Q.hl) ? 0 : (el == Q.EX + 1 && !Q.hr) ? L.Rm : -1;
   const int w_lo = warp > 0 ? s_wo[warp - 1] : 0, w_hi = s_wo[warp];  // exchange words this warp sends
   const int oc = N * L.Wp + off + N + ec * N;   // region offset of the column's first owned node
 
@@ -825,16 +822,18 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
             SX[j][i] = __ffma2_rn(make_float2(tz[j].z, tz[j].w), SX[j][i], __fmul2_rn(Rx[i], SZr[j][i]));  // sens_increment
         if (stc_edge && t <= S.nt - 2 && mine) {
           // g lambda (b_{t+2} - b_t) at the absorbing edges, rounded as bnd_sens
+          auto sens = [&](int j, int i, int k) {
+            float& f = (i & 1) ? SX[j][i / 2].y : SX[j][i / 2].x;
+            f = __fadd_rn(f, __fmul_rn(__fmul_rn(sm[L.be + 2 * bn + k], lane_of(xu[j], i)), sm[L.bd + (t & 1) * bn + k]));
+          };
 #pragma unroll
           for (int j = 0; j < NJ; ++j)
+            if (side >= 0 && r0 + j < Q.R && Q.gz0 + r0 + j > 0) sens(j, 0, side + r0 + j);
+          if (vz && h == 0) {
 #pragma unroll
-            for (int i = 0; i < N; ++i) {
-              const int k = edge_of(r0 + j, ec * N + i);
-              if (k >= 0) {
-                float& f = (i & 1) ? SX[j][i / 2].y : SX[j][i / 2].x;
-                f = __fadd_rn(f, __fmul_rn(__fmul_rn(sm[L.be + 2 * bn + k], lane_of(xu[j], i)), sm[L.bd + (t & 1) * bn + k]));
-              }
-            }
+            for (int i = 0; i < N; ++i)
+              if (ec * N + i < Q.C && !(i == 0 && side >= 0)) sens(0, i, 2 * L.Rm + ec * N + i);
+          }
         }
 #pragma unroll
         for (int j = 0; j < NJ; ++j)
@@ -843,31 +842,62 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
         if (mine) vg_put(g, L.g, S.grad);
       }
       if constexpr (!VG) vg_get(v, L.v, nullptr);
-      if constexpr (STC) {
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < H2; ++i)
+          X[j][i] = __ffma2_rn(make_float2(tz[j].z, tz[j].w), X[j][i], __fmul2_rn(Rx[i], Zr[j][i]));
+      if (ADJ && niq > 0 && mine) {
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-          const int r = r0 + j;
-          const bool top = Q.gz0 + r == 0;
-          int m = 0;
-          if (ADJ && niq > 0 && mine) m = imap[r * L.qx + ec];
+          const int m = imap[(r0 + j) * L.qx + ec];
+          if (m) {  // P (injection - K) + mu
+            const float* ex = sm + L.ia + (t & 1) * (L.niq * N) + (m - 1) * N;
 #pragma unroll
-          for (int i = 0; i < N; ++i) {
-            float e1 = 1.f, e2 = 1.f;
-            int k = -1;
-            if (stc_edge && mine) {
-              k = edge_of(r, ec * N + i);
-              if (k >= 0) { e1 = sm[L.be + k]; e2 = sm[L.be + bn + k]; }
+            for (int i = 0; i < N; ++i) {
+              float& k = (i & 1) ? X[j][i / 2].y : X[j][i / 2].x;
+              k = -__fsub_rn(ex[i], k);
             }
-            float ex = 0.f;
-            if (!ADJ) { if (r == src_r && ec == src_e && i == src_i) ex = s_src[t & 1]; }
-            else if (m) ex = sm[L.ia + (t & 1) * (L.niq * N) + (m - 1) * N + i];
-            float rr, vv;
-            advance_node_stacey(ADJ, lane_of(xu[j], i), lane_of(v[j], i), lane_of(X[j], i), lane_of(Zr[j], i), -lane_of(nix, i),
-                                lane_of(Rx, i), tz[j].x, tz[j].z, ex, e1, e2, rr, vv);
-            if (top) { rr = 0.f; vv = 0.f; }
-            if (i & 1) { X[j][i / 2].y = rr; v[j][i / 2].y = vv; } else { X[j][i / 2].x = rr; v[j][i / 2].x = vv; }
-            if (!ADJ && k >= 0 && keep)
-              S.bnd_hist[(long long)(t + 1) * S.bnd_pitch + bnd_slot(S, Q.gx0 + ec * N + i, Q.gz0 + r)] = rr;
+          }
+        }
+      }
+      const bool here = !ADJ && src_r >= r0 && src_r < r0 + NJ && ec == src_e;  // the source's quad
+      if constexpr (STC) {
+        // as advance_node_stacey, two nodes at a time: w = v + F, and at the absorbing edges w = e1 v + e2 F
+        const bool bottom = vz && h == 0 && mine && stc_edge, top = Q.gz0 + r0 == 0;
+        const float* const be = sm + L.be;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const int ks = side >= 0 && mine && r0 + j < Q.R ? side + r0 + j : -1;
+#pragma unroll
+          for (int i = 0; i < H2; ++i) {
+            const float2 np = __fmul2_rn(nix[i], make_float2(tz[j].x, tz[j].y));
+            float2 f = ADJ ? __fmul2_rn(np, X[j][i]) : __ffma2_rn(np, X[j][i], make_float2(0.f, 0.f));
+            if (here && r0 + j == src_r) {
+              if (src_i == 2 * i) f.x = __fmaf_rn(np.x, X[j][i].x, s_src[t & 1]);
+              if (src_i == 2 * i + 1) f.y = __fmaf_rn(np.y, X[j][i].y, s_src[t & 1]);
+            }
+            float2 w = make_float2(__fadd_rn(v[j][i].x, f.x), __fadd_rn(v[j][i].y, f.y));
+            if (i == 0 && ks >= 0) w.x = __fmaf_rn(be[ks], v[j][i].x, __fmul_rn(be[bn + ks], f.x));
+            if (j == 0 && bottom) {
+              const int c0 = ec * N + 2 * i, k = 2 * L.Rm + c0;
+              if (c0 < Q.C && !(i == 0 && side >= 0)) w.x = __fmaf_rn(be[k], v[j][i].x, __fmul_rn(be[bn + k], f.x));
+              if (2 * i + 1 < N && c0 + 1 < Q.C) w.y = __fmaf_rn(be[k + 1], v[j][i].y, __fmul_rn(be[bn + k + 1], f.y));
+            }
+            if (j == 0 && top) w = make_float2(0.f, 0.f);
+            X[j][i] = j == 0 && top ? w : __fadd2_rn(xu[j][i], w);
+            v[j][i] = w;
+          }
+        }
+        if (!ADJ && keep && stc_edge && mine) {
+          float* const hist = S.bnd_hist + (long long)(t + 1) * S.bnd_pitch;
+#pragma unroll
+          for (int j = 0; j < NJ; ++j)
+            if (side >= 0 && r0 + j < Q.R && Q.gz0 + r0 + j > 0) hist[(side ? S.nzg : 0) + Q.gz0 + r0 + j] = X[j][0].x;
+          if (bottom) {
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+              if (ec * N + i < Q.C && !(i == 0 && side >= 0)) hist[2 * S.nzg + Q.gx0 + ec * N + i] = lane_of(X[0], i);
           }
         }
       } else {
@@ -876,27 +906,8 @@ __global__ void __launch_bounds__(res_threads(LPE, ADJ), 1)
         for (int j = 0; j < NJ; ++j)
 #pragma unroll
           for (int i = 0; i < H2; ++i)
-            X[j][i] = __ffma2_rn(make_float2(tz[j].z, tz[j].w), X[j][i], __fmul2_rn(Rx[i], Zr[j][i]));
-        if (ADJ && niq > 0 && mine) {
-#pragma unroll
-          for (int j = 0; j < NJ; ++j) {
-            const int m = imap[(r0 + j) * L.qx + ec];
-            if (m) {  // P (injection - K) + mu
-              const float* ex = sm + L.ia + (t & 1) * (L.niq * N) + (m - 1) * N;
-#pragma unroll
-              for (int i = 0; i < N; ++i) {
-                float& k = (i & 1) ? X[j][i / 2].y : X[j][i / 2].x;
-                k = -__fsub_rn(ex[i], k);
-              }
-            }
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < NJ; ++j)
-#pragma unroll
-          for (int i = 0; i < H2; ++i)
             v[j][i] = __ffma2_rn(__fmul2_rn(nix[i], make_float2(tz[j].x, tz[j].y)), X[j][i], v[j][i]);
-        if (!ADJ && src_r >= r0 && src_r < r0 + NJ && ec == src_e) {
+        if (here) {
           const float s = s_src[t & 1];
 #pragma unroll
           for (int j = 0; j < NJ; ++j)

@@ -169,7 +169,7 @@ bool res_shape(int N, int vr, bool adj, int exm, int ezm, int ezl, int nrec, Res
   const int ezr = std::max(ezm, ezl + 1);  // element rows, the mesh's last line of nodes counted as one
   h->nio = (int)round_up(std::max(nrec, 1), 32);
   h->edge = (exm + ezm) * N * (N + 1);
-  const int tmax = res_threads(res_lanes(vr), adj) - h->nio;
+  const int tmax = res_threads(N, res_lanes(vr), adj) - h->nio;
   h->sw = 4;
   while (h->sw < (exm + 2) * res_lanes(vr)) h->sw *= 2;
   if (h->sw > 32 || tmax < 32) return false;
