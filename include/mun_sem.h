@@ -218,19 +218,22 @@ int sem_forward_noalloc(const sem_plan_t* plan, const double* velocity, float* r
 /* ---------------------------------------------------------------------------------
  * Serving engine: continuous batching (no counterpart in the reference, whose
  * drivers call SEMSimulation one request at a time: MCMC.py:193-208,
- * RQS_Coupling.py:295-351).  Solves are queued with sem_engine_submit and admitted at
- * the next tick boundary when a slot and enough device memory (the solve's workspace
- * under memory_cap) are free; each sem_engine_step retires finished solves, admits
- * queued ones and launches ticks_per_step ticks on the stream.  A solve's results do
- * not depend on what runs beside it (bitwise).  One thread uses an engine at a time.
+ * RQS_Coupling.py:295-351).  Solves are queued with sem_engine_submit and admitted in
+ * order of arrival by sem_engine_step when a slot and enough device memory (the solve's
+ * workspace under memory_cap) are free.  With kernel and tile automatic, solves that fit
+ * the SMs run whole, all that a step admits (up to 40 ms of modelled work) as one march
+ * of the resident kernels, while at most one earlier march is unfinished on the stream.
+ * The others (too large, longer than that, or with a kernel or tile given) run side by
+ * side by ticks, ticks_per_step with each call.  A solve's results do not depend on what
+ * runs beside it (bitwise).  One thread uses an engine at a time.
  * ------------------------------------------------------------------------------- */
 typedef struct sem_engine_s sem_engine_t;
 typedef struct {
   int32_t max_solves;      /* concurrent solves                                        */
   int64_t memory_cap;      /* device bytes for solve workspaces (allocated at creation) */
   int32_t ticks_per_step;  /* ticks launched by one sem_engine_step                    */
-  int32_t kernel;          /* 0 automatic per step (as in sem_run), 1 tile kernel,
-                              2 strip kernel                                           */
+  int32_t kernel;          /* 0 automatic per step (as in sem_run: resident marches, or
+                              ticks of strips or tiles), 1 tile kernel, 2 strip kernel */
   int32_t tile_ex, tile_ez;/* tile kernel tile size; 0 x 0 = automatic per step        */
 } sem_engine_cfg_t;
 
@@ -239,13 +242,14 @@ int sem_engine_destroy(sem_engine_t* engine);
 /* queue one solve (same fields as in sem_run; its buffers must stay valid until it is
  * released) and return a ticket */
 int sem_engine_submit(sem_engine_t* engine, const sem_solve_t* solve, int64_t* ticket);
-/* retire, admit, launch ticks_per_step ticks */
+/* retire, admit, launch a march of what fits the SMs and ticks_per_step ticks of the rest */
 int sem_engine_step(sem_engine_t* engine, void* stream);
 /* *state: 0 queued, 1 running, 2 done (outputs written), -1 unknown ticket */
 int sem_engine_status(sem_engine_t* engine, int64_t ticket, int32_t* state);
 /* forget a done solve */
 int sem_engine_release(sem_engine_t* engine, int64_t ticket);
-/* out[5]: queued, running, workspace bytes in use, ticks launched, kernel launches */
+/* out[5]: queued, running (workspace held), workspace bytes in use, ticks launched, kernel
+ * launches */
 int sem_engine_stats(const sem_engine_t* engine, int64_t* out);
 
 /* ---------------------------------------------------------------------------------

@@ -45,6 +45,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <deque>
 #include <map>
@@ -3171,7 +3172,7 @@ int sem_run(sem_batch_t* b, const sem_solve_t* solves, int32_t n, const sem_laun
   std::vector<sem_solve_t> left;
   if (resident) {
     std::vector<int> rest;
-    if (int rc = run_resident(b, solves, n, budget, stream, &rest)) return rc;
+    if (int rc = run_resident(b, solves, nullptr, n, budget, stream, &rest)) return rc;
     if (rest.empty()) return SEM_OK;
     if (cfg.kernel == 5) cfg.kernel = 0;
     for (int i : rest) left.push_back(solves[i]);
@@ -3370,12 +3371,14 @@ int sem_forward_adjoint(sem_batch_t* b, const sem_plan_t* plan, const double* ve
 }  // extern "C"
 
 // ============================================================================
-// serving engine: continuous batching over the tick program
+// serving engine: continuous batching over resident marches and the tick program
 // ============================================================================
 struct EngineJob {
   sem_solve_t s{};
   int64_t ticket = 0;
   int k = 2, nseg = 1, prog = 0, ntiles = 0, state = 0;  // 0 queued, 1 running, 2 retired
+  int march = 0;          // runs resident: 1 forward, 2 with the adjoint
+  double share = 0.0;     // ns of the SMs' time its march takes
   long long start = 0, off = -1;
   Workspace ws{};
   cudaEvent_t ev = nullptr;
@@ -3408,9 +3411,29 @@ struct sem_engine_s {
   CUtensorMap* d_tmaps = nullptr;
   int tmaps_cap = 0;
   std::vector<CUtensorMap> h_tmaps;
+  sem_batch_t* res = nullptr;          // descriptors and exchange words of the resident marches
+  std::vector<EngineJob*> marched;     // their solves whose workspaces are still held
+  std::deque<cudaEvent_t> marches;     // ends of the marches on the stream, oldest first
 };
 
 namespace {
+
+// What one step admits to the resident kernels, in ns of modelled march, and the marches that may be
+// unfinished on the stream when a step adds one: a request waits for at most these before its own
+// (a longer solve than one step's share runs by ticks, beside the others).  A second march keeps
+// the GPU busy while the host sees the first one's end.  (16 likelihoods of 80x40 and less and 8
+// gradients of 80x40, 600 to 720 steps: 18.2 ms by ticks, 7.8 marched.)
+constexpr double kMarchNs = 40e6;
+constexpr size_t kMarches = 2;
+// ns of a solve's march: its share of full SMs (measured on 128 models of 100x50: 4.5 ps a node and
+// step forward, 12.5 with the adjoint), and alone (2 and 4 us a step of 100x50)
+void march_ns(const sem_solve_t& s, int k, int nseg, double* share, double* alone) {
+  const sem_plan_s* p = s.plan;
+  const bool adj = s.flags & SEM_F_ADJOINT;
+  const double fwd = (double)p->nt + (adj ? (double)k * (nseg - 1) : 0.0), back = adj ? (double)p->nt : 0.0;
+  *share = (4.5e-3 * fwd + 8e-3 * back) * (double)p->npoints;
+  *alone = std::max(*share, 2000.0 * (fwd + back));
+}
 
 // set-up / output table entry of one solve whose workspace starts at `a`
 SolveIo solve_io(const sem_solve_t& s, const Workspace& ws, char* a) {
@@ -3477,6 +3500,66 @@ void arena_free(sem_engine_s* e, long long off, long long bytes) {
   }
 }
 
+// workspaces of marched solves back to the arena: all of them (the stream orders later work behind
+// the marches) or those that have ended
+void free_marched(sem_engine_s* e, bool all) {
+  size_t keep = 0;
+  for (EngineJob* j : e->marched) {
+    if (all || cudaEventQuery(j->ev) == cudaSuccess) arena_free(e, j->off, j->ws.bytes);
+    else e->marched[keep++] = j;
+  }
+  e->marched.resize(keep);
+}
+
+// Launches the admitted solves that run resident, forward ones first (their results are due first), and
+// leaves the others, in their order, in `admitted`.
+int engine_march(sem_engine_s* e, std::vector<EngineJob*>* admitted, cudaStream_t stream) {
+  if (!e->res)
+    if (int rc = sem_batch_create(&e->res)) return rc;
+  sem_batch_t* b = e->res;
+  std::vector<char> done(admitted->size(), 0);
+  for (int adj = 0; adj < 2; ++adj) {
+    std::vector<size_t> of;
+    std::vector<sem_solve_t> sv;
+    std::vector<char*> at;
+    for (size_t i = 0; i < admitted->size(); ++i) {
+      EngineJob* j = (*admitted)[i];
+      if (j->march != (adj ? 2 : 1)) continue;
+      of.push_back(i);
+      sv.push_back(j->s);
+      sv.back().ckpt_k = j->k;
+      at.push_back(e->arena + j->off);
+    }
+    if (of.empty()) continue;
+    b->last_launches = 0;
+    b->tick_ev_used = 0;
+    std::vector<int> rest;
+    // (no budget: the workspaces are there)
+    if (int rc = run_resident(b, sv.data(), at.data(), (int)sv.size(), LLONG_MAX / 2, stream, &rest)) return rc;
+    e->launches += b->last_launches;
+    for (size_t i = 0; i < of.size(); ++i) {
+      if (std::find(rest.begin(), rest.end(), (int)i) != rest.end()) continue;
+      EngineJob* j = (*admitted)[of[i]];
+      CUDA_TRY(cudaEventCreateWithFlags(&j->ev, cudaEventDisableTiming));
+      CUDA_TRY(cudaEventRecord(j->ev, stream));
+      j->state = 2;
+      e->marched.push_back(j);
+      done[of[i]] = 1;
+    }
+  }
+  size_t keep = 0;
+  for (size_t i = 0; i < admitted->size(); ++i)
+    if (!done[i]) (*admitted)[keep++] = (*admitted)[i];
+  if (keep < admitted->size()) {
+    cudaEvent_t ev;
+    CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    e->marches.push_back(ev);
+    CUDA_TRY(cudaEventRecord(ev, stream));
+  }
+  admitted->resize(keep);
+  return SEM_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -3516,6 +3599,8 @@ int sem_engine_destroy(sem_engine_t* e) {
   }
   cudaFree(e->arena); cudaFree(e->d_tick); cudaFree(e->d_solves); cudaFree(e->d_cta); cudaFree(e->d_tmaps);
   cudaFree(e->d_io);
+  for (cudaEvent_t ev : e->marches) cudaEventDestroy(ev);
+  sem_batch_destroy(e->res);
   delete e;
   return SEM_OK;
 }
@@ -3540,6 +3625,13 @@ int sem_engine_submit(sem_engine_t* e, const sem_solve_t* s, int64_t* ticket) {
   }
   const int nt = s->plan->nt;
   j->prog = nt + ((s->flags & SEM_F_SHIFT) ? 1 : 0) + (adj ? 1 + nt + j->k * (j->nseg - 1) : 0);
+  if (e->cfg.kernel == 0 && e->cfg.tile_ex == 0) {
+    double alone;
+    march_ns(*s, j->k, j->nseg, &j->share, &alone);
+    sem_solve_t t = *s;
+    t.ckpt_k = j->k;
+    if (alone <= kMarchNs && res_class(t, sm_count(e->device))) j->march = adj ? 2 : 1;
+  }
   e->queue.push_back(j);
   e->jobs[j->ticket] = j;
   *ticket = j->ticket;
@@ -3555,6 +3647,7 @@ int sem_engine_status(sem_engine_t* e, int64_t ticket, int32_t* state) {
   const cudaError_t q = cudaEventQuery(j->ev);
   if (q == cudaErrorNotReady) { *state = 1; return SEM_OK; }
   CUDA_TRY(q);
+  if (j->march) free_marched(e, false);
   *state = 2;
   return SEM_OK;
 }
@@ -3567,6 +3660,7 @@ int sem_engine_release(sem_engine_t* e, int64_t ticket) {
   if (j->state != 2) return fail(SEM_ERR_ARG, "solve still queued or running");
   if (j->ev) {
     CUDA_TRY(cudaEventSynchronize(j->ev));
+    if (j->march) free_marched(e, false);
     cudaEventDestroy(j->ev);
   }
   delete j;
@@ -3577,7 +3671,7 @@ int sem_engine_release(sem_engine_t* e, int64_t ticket) {
 int sem_engine_stats(const sem_engine_t* e, int64_t* out) {
   if (!e || !out) return fail(SEM_ERR_ARG, "null argument");
   out[0] = (int64_t)e->queue.size();
-  out[1] = (int64_t)e->running.size();
+  out[1] = (int64_t)(e->running.size() + e->marched.size());
   out[2] = e->in_use;
   out[3] = e->tick;
   out[4] = e->launches;
@@ -3605,29 +3699,36 @@ int sem_engine_step(sem_engine_t* e, void* stream_v) {
   // workspaces may reuse the retiring solves' memory: the set-up launch follows the
   // output launch on the stream)
   for (EngineJob* j : retiring) arena_free(e, j->off, j->ws.bytes);
+  while (!e->marches.empty() && cudaEventQuery(e->marches.front()) == cudaSuccess) {
+    cudaEventDestroy(e->marches.front());
+    e->marches.pop_front();
+  }
+  const bool march = e->marches.size() < kMarches;
+  free_marched(e, march && !e->queue.empty());
+  double share = 0.0;
   std::vector<EngineJob*> admitted;
-  while (!e->queue.empty() && (int)e->running.size() < e->cfg.max_solves) {
+  while (!e->queue.empty() && (int)(e->running.size() + e->marched.size() + admitted.size()) < e->cfg.max_solves) {
     EngineJob* j = e->queue.front();
+    if (j->march && (!march || (share > 0.0 && share + j->share > kMarchNs))) break;
     const long long off = arena_alloc(e, j->ws.bytes);
     if (off < 0) break;
     e->queue.pop_front();
     j->off = off;
     j->start = e->tick;
     j->state = 1;
-    e->h_io.push_back(solve_io(j->s, j->ws, e->arena + off));
+    if (j->march) share += j->share;
     admitted.push_back(j);
-    e->running.push_back(j);
   }
-  const int nadm = (int)e->h_io.size() - nret;
-  if (!e->h_io.empty())
-    CUDA_TRY(cudaMemcpyAsync(e->d_io, e->h_io.data(), sizeof(SolveIo) * e->h_io.size(),
-                             cudaMemcpyHostToDevice, stream));
   auto io_blocks = [&](int s0, int cnt) {
     long long mx = 1;
     for (int i = s0; i < s0 + cnt; ++i) mx = std::max(mx, (long long)e->h_io[i].npoints);
     return (unsigned)std::min<long long>(64, (mx + 2047) / 2048);
   };
+  auto io_copy = [&](int s0, int cnt) {
+    return cudaMemcpyAsync(e->d_io + s0, e->h_io.data() + s0, sizeof(SolveIo) * cnt, cudaMemcpyHostToDevice, stream);
+  };
   if (nret > 0) {
+    CUDA_TRY(io_copy(0, nret));
     batch_output_kernel<<<dim3(io_blocks(0, nret), (unsigned)nret), 256, 0, stream>>>(e->d_io, 0);
     e->launches++;
     for (EngineJob* j : retiring) {
@@ -3636,7 +3737,18 @@ int sem_engine_step(sem_engine_t* e, void* stream_v) {
       j->state = 2;
     }
   }
+  // ---- solves that fit on chip march at once, on the stream behind the outputs above
+  if (std::any_of(admitted.begin(), admitted.end(), [](EngineJob* j) { return j->march > 0; }))
+    if (int rc = engine_march(e, &admitted, stream)) return rc;
+  // ---- the others run by ticks from here
+  const int nadm = (int)admitted.size();
+  for (EngineJob* j : admitted) {
+    j->march = 0;
+    e->h_io.push_back(solve_io(j->s, j->ws, e->arena + j->off));
+    e->running.push_back(j);
+  }
   if (nadm > 0) {
+    CUDA_TRY(io_copy(nret, nadm));
     batch_setup_kernel<<<dim3(io_blocks(nret, nadm), (unsigned)nadm), 256, 0, stream>>>(e->d_io, nret);
     e->launches++;
   }

@@ -434,9 +434,9 @@ struct ResWave {
   const std::vector<int>* solves;
 };
 
-// One group: set-up, forward launches, (replay and) adjoint launches, outputs.
-// SEM_ERR_UNSUPPORTED without a message when the group cannot run this way (nothing launched).
-int run_res_group(sem_batch_t* b, const sem_solve_t* sv, const ResGroup& w, int sms, cudaStream_t stream) {
+// One group: set-up, forward launches, (replay and) adjoint launches, outputs.  at: the solves'
+// workspaces, or null (the batch's arena).  SEM_ERR_UNSUPPORTED without a message when the group cannot run this way (nothing launched).
+int run_res_group(sem_batch_t* b, const sem_solve_t* sv, char* const* at, const ResGroup& w, int sms, cudaStream_t stream) {
   const int n = (int)w.idx.size();
   const sem_plan_s* p0 = sv[w.idx[0]].plan;
   const int N = p0->npol;
@@ -499,7 +499,7 @@ int run_res_group(sem_batch_t* b, const sem_solve_t* sv, const ResGroup& w, int 
     total += ws[j].bytes;
     max_seg = std::max(max_seg, nseg[j]);
   }
-  if (total > b->arena_bytes) {
+  if (!at && total > b->arena_bytes) {
     cudaFree(b->arena);
     b->arena = nullptr;
     b->arena_bytes = 0;
@@ -522,7 +522,7 @@ int run_res_group(sem_batch_t* b, const sem_solve_t* sv, const ResGroup& w, int 
   for (int j = 0; j < n; ++j) {
     const sem_solve_t& s = sv[w.idx[j]];
     const sem_plan_s* p = s.plan;
-    char* a = b->arena + off;
+    char* a = at ? at[w.idx[j]] : b->arena + off;
     SolveDev& d = b->h_solves[j];
     d.nelx = p->nelx; d.nelz = p->nelz; d.nxg = p->nxg; d.nzg = p->nzg; d.pitch = p->pitch;
     d.tiles_x = w.fwd.tiles[j].tx; d.tiles_z = w.fwd.tiles[j].tz;
@@ -685,26 +685,35 @@ int run_res_group(sem_batch_t* b, const sem_solve_t* sv, const ResGroup& w, int 
   return SEM_OK;
 }
 
-// Runs what can run resident and returns the solves that cannot in `rest`.
-int run_resident(sem_batch_t* b, const sem_solve_t* sv, int n, long long budget, cudaStream_t stream,
-                 std::vector<int>* rest) {
+int sm_count(int device) {
   int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  return sms;
+}
+// The class a solve runs resident in, or 0.  Adjoint solves too large for shared memory that were
+// given a checkpoint interval keep the strip kernel, whose schedule the interval was chosen for.
+int res_class(const sem_solve_t& s, int sms) {
+  const int need = res_need(s.plan, s.flags & SEM_F_ADJOINT, sms);
+  return need == RES_MEM && s.ckpt_k > 0 && s.ckpt_k < s.plan->nt ? 0 : need;
+}
+
+// Runs what can run resident and returns the solves that cannot in `rest`.  at: see run_res_group.
+int run_resident(sem_batch_t* b, const sem_solve_t* sv, char* const* at, int n, long long budget, cudaStream_t stream,
+                 std::vector<int>* rest) {
+  const int sms = sm_count(b->device);
   std::map<std::tuple<int, bool, bool, int>, std::vector<int>> classes;
   for (int i = 0; i < n; ++i) {
     const sem_plan_s* p = sv[i].plan;
     const bool adj = sv[i].flags & SEM_F_ADJOINT;
-    const int need = res_need(p, adj, sms);
-    // adjoint solves too large for shared memory that were given a checkpoint interval keep the strip
-    // kernel, whose schedule the interval was chosen for
-    if (!need || (need == RES_MEM && sv[i].ckpt_k > 0 && sv[i].ckpt_k < p->nt)) rest->push_back(i);
+    const int need = res_class(sv[i], sms);
+    if (!need) rest->push_back(i);
     else classes[std::make_tuple(p->npol, p->bnd_n > 0, adj, need)].push_back(i);
   }
   for (auto& kv : classes) {
     const std::vector<ResGroup> groups = res_plan(sv, kv.second, sms, budget);
     if (groups.empty()) { rest->insert(rest->end(), kv.second.begin(), kv.second.end()); continue; }
     for (const ResGroup& g : groups) {
-      const int rc = run_res_group(b, sv, g, sms, stream);
+      const int rc = run_res_group(b, sv, at, g, sms, stream);
       if (rc == SEM_ERR_UNSUPPORTED) rest->insert(rest->end(), g.idx.begin(), g.idx.end());
       else if (rc) return rc;
     }

@@ -2,10 +2,12 @@
 
 Requests are forward-only likelihoods (MCMC proposals: forward with the misfit summed on
 the device) and forward+adjoint gradients (flow-trainer samples).  The engine keeps
-every admitted solve's wavefields and checkpoints resident in its arena and admits a
-queued request at the next tick boundary as soon as a slot and enough device memory
-(its workspace footprint, under the engine's byte cap) are free, so requests that
-arrive while others run overlap with them on the device.  Each solve's result is
+every admitted solve's wavefields and checkpoints in its arena and admits queued
+requests in order of arrival as soon as a slot and enough device memory (a solve's
+workspace footprint, under the engine's byte cap) are free.  Requests that fit the SMs
+are marched whole by the resident kernels, all that wait at a step together; those that
+arrive meanwhile form the next march.  Larger or very long ones advance by ticks, side
+by side, and overlap on the device with those that arrive later.  Each solve's result is
 bitwise identical alone and in any mix (deterministic kernels, per-solve time
 program).
 """
@@ -27,7 +29,8 @@ class Engine:
 
     def __init__(self, max_solves=512, memory_cap_bytes=8 << 30, ticks_per_step=16, kernel=0,
                  tile=(0, 0), stream=None):
-        """kernel 0 / tile (0, 0): chosen per step for the running set (as in sem_run)."""
+        """kernel 0 / tile (0, 0): resident marches where they fit; else chosen per step for the
+        running set (as in sem_run)."""
         lib = _lib.load()
         cfg = _lib.EngineCfg(int(max_solves), int(memory_cap_bytes), int(ticks_per_step), int(kernel),
                              int(tile[0]), int(tile[1]))

@@ -81,3 +81,32 @@ def test_request_loop_poisson_stream():
     assert np.all(lat > 0)
     print(f"served {len(done)} requests in {wall:.3f} s, p50 {1e3 * np.percentile(lat, 50):.1f} ms, "
           f"p99 {1e3 * np.percentile(lat, 99):.1f} ms")
+
+
+def test_engine_marches_beside_ticks():
+    # a solve too long for one march runs by ticks beside marched ones, whose workspaces are reused
+    # by the next march while the last one may still run
+    g = load(INJECT[0])
+    y, v = dev(aligned_obs(g)), np.asarray(g["velocity"])
+    inv = 1.0 / float(g["sigma"]) ** 2
+    short, long_ = plan_for(g["config"], g["dt"], g["nt"]), plan_for(g["config"], g["dt"], 20100)
+
+    def make(i):
+        if i == 3:
+            return SolveSpec(long_, dev(v))
+        return SolveSpec(short, dev(v * (1.0 + 0.003 * i)), adjoint=i % 2 == 0, misfit=True, y_obs=y, inv_sigma2=inv,
+                         shift=True, ckpt_k=(0, 7)[i % 4 == 0])
+    alone = [make(i) for i in range(12)]
+    for s in alone:
+        Batch().run([s])
+    one = max(s.plan.workspace_bytes(s.flags, s.ckpt_k or s.plan.nt) for s in alone)
+    eng = Engine(max_solves=5, memory_cap_bytes=max(1 << 20, int(3.5 * one)), ticks_per_step=64)
+    tickets = [eng.submit(make(i)) for i in range(12)]
+    eng.run_until_done(tickets)
+    for t, a in zip(tickets, alone):
+        b = eng.release(t)
+        assert int(b.status.item()) == 0
+        assert torch.equal(a.rec, b.rec)
+        assert a.loglik is None or torch.equal(a.loglik, b.loglik)
+        assert a.grad is None or torch.equal(a.grad, b.grad)
+    assert eng.stats()["bytes_in_use"] == 0 and eng.stats()["running"] == 0
