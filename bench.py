@@ -47,6 +47,8 @@ BYTES_PER_NODE_ADJ_TICK = 36
 # b, v); adjoint tick 32.5 (reads lambda, mu, c^2 and the forward b, writes lambda and mu,
 # float32 partial gradient read-modify-write, and a float64 fold every 16 ticks)
 IMPL_BYTES_PER_NODE = {"forward_tick": 20, "adjoint_tick": 32.5}
+# and the resident kernels: the forward history written and read, a float64 fold every 16 steps
+RESIDENT_BYTES_PER_NODE = {"forward_step": 4, "adjoint_step": 5}
 # DRAM bytes per node and tick of the strip kernel from one ncu capture (dram__bytes_read +
 # dram__bytes_write of one forward and one adjoint tick of a 128-model group, 10.3 M nodes),
 # scaled to a launch by its nodes
@@ -781,9 +783,10 @@ def main():
     barrier()
     ms = float(np.mean(step_ms))
     ticks_per_step = batch.last_ticks
+    resident = kernel_used == "resident"  # its launches march many steps; it counts waves as groups
     # node-ticks of each kind per step: every group runs nt adjoint ticks, a read-out and
     # a scale tick; its remaining ticks are forward or replay ticks
-    fwd_like = ticks_per_step - groups_used * (W["nt"] + 2)
+    fwd_like = None if resident else ticks_per_step - groups_used * (W["nt"] + 2)
     # algorithmic bytes of the step's tick launches: 56 B per node-step (replay ticks are
     # overhead and carry none)
     kern_bytes = BYTES_PER_NODE_STEP_FWDADJ * W["npoints"] * W["nt"] * n
@@ -911,13 +914,15 @@ def main():
                          "bytes_per_node_step": BYTES_PER_NODE_STEP_FWDADJ,
                          "bytes_per_node": {"forward_tick": BYTES_PER_NODE_FWD_TICK,
                                             "adjoint_tick": BYTES_PER_NODE_ADJ_TICK},
-                         "kernel_bytes_per_node": IMPL_BYTES_PER_NODE,
+                         "kernel_bytes_per_node": RESIDENT_BYTES_PER_NODE if resident else IMPL_BYTES_PER_NODE,
+                         # resident: a wave's step
                          "launch_us_avg": 1e3 * tick_loop_ms / ticks_per_step,
                          "ticks_per_step": ticks_per_step, "forward_like_ticks": fwd_like,
                          "note": "algorithmic bytes (56 per fwd+adj node-step) of the step's tick "
-                                 "launches over the CUDA-event time of the tick loops (one "
-                                 "tick-kernel launch per tick, chained by programmatic dependent "
-                                 "launch); traffic = ncu DRAM bytes per launch",
+                                 "launches over the CUDA-event time of the tick loops (resident "
+                                 "kernels: one launch per wave of solves and sweep, state on chip; "
+                                 "tick kernels: one launch per tick, traffic = ncu DRAM bytes per "
+                                 "launch)",
                          "step_level": {"bytes_per_node_step": BYTES_PER_NODE_STEP_FWDADJ,
                                         "achieved": step_achieved,
                                         "frac": step_achieved / peak}},

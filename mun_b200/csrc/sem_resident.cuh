@@ -21,6 +21,10 @@
 // later, after words that its readers sent when they were done with it (two steps
 // suffice for direct neighbours, three for the corner node).
 //
+// Clusters.  A solve of at most 16 tiles can be one thread-block cluster: the words then go straight
+// into the neighbours' shared memory and are polled there, without the way through L2, and no
+// cooperative launch is needed (solves do not wait for one another).
+//
 // Threads.  A compute thread owns a column of elements, or of their halves: lane by lane the
 // elements of a tile row, stepping down the element rows of its chunk.  All lines of an element
 // are evaluated in registers; the carry into the element below stays in registers, the carry into
@@ -63,6 +67,7 @@ struct ResLay {
   int nrm, niq, Rm, Cm;          // most receivers and injection quads per tile, owned rows, columns
   int total;                     // floats
   int llw, ll_t, ll_r, ll_b, ll_c;  // exchange words per CTA and slot; offsets of the sides
+  int sl;                        // clusters: the slots of arriving words; -1: they are in memory
 };
 
 enum : int { RES_FWD = 0, RES_REPLAY = 1, RES_ADJ = 2 };
@@ -75,6 +80,20 @@ __device__ __forceinline__ unsigned long long ll_load(const unsigned long long* 
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
+}
+// the same between the CTAs of a cluster: shared-memory address p of CTA `rank`, and of this CTA
+__device__ __forceinline__ void ll_send_cluster(unsigned p, int rank, float v, unsigned tag) {
+  const unsigned long long q = ((unsigned long long)tag << 32) | (unsigned long long)__float_as_uint(v);
+  asm volatile("{ .reg .u32 a; mapa.shared::cluster.u32 a, %0, %1; st.relaxed.cluster.shared::cluster.u64 [a], %2; }"
+               ::"r"(p), "r"(rank), "l"(q) : "memory");
+}
+__device__ __forceinline__ unsigned long long ll_load_shared(unsigned p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 // Exchange words' table entries.  In: place in this CTA's slot and region index.  Out: place among
@@ -240,10 +259,10 @@ __device__ __forceinline__ void res_xline(const float (&u)[N + 1], const float (
   }
 }
 
-// nc: compute threads (the first of the CTA); the rest serve the receivers.  sw: lanes per tile
+// CL: the solve's tiles are one cluster.  nc: compute threads (the first of the CTA); the rest serve the receivers.  sw: lanes per tile
 // row (a power of two, at least the tile's columns of elements + 2: one for the left halo, one
 // for the nodes on the right); ezc: element rows per chunk.
-template <int N, int LPE, bool ADJ, bool STC, bool VG>
+template <int N, int LPE, bool ADJ, bool STC, bool VG, bool CL>
 __global__ void __launch_bounds__(res_threads(N, LPE, ADJ), 1)
     sem_resident_kernel(const SolveDev* __restrict__ solves, const int* __restrict__ cta_solve,
                         const __grid_constant__ ResLay L, unsigned long long* __restrict__ ll,
@@ -253,6 +272,7 @@ __global__ void __launch_bounds__(res_threads(N, LPE, ADJ), 1)
   // two lanes per element (order 4): each has two columns' z-lines and two rows' x-lines and nodes
   static_assert(LPE == 1 || N == 4, "an element's halves");
   static_assert(!VG || (ADJ && LPE == 1), "large adjoint tiles");
+  static_assert(!VG || !CL, "a cluster's tiles are small");  // (a switch at run time cost two lanes forward 4 %)
   constexpr int NJ = N / LPE, NQ = LPE == 2 ? 1 : H2;
   extern __shared__ __align__(128) float sm[];
   __shared__ SolveDev S;
@@ -326,6 +346,7 @@ __global__ void __launch_bounds__(res_threads(N, LPE, ADJ), 1)
       }
   }
   // ---------------- exchange words that arrive
+  const unsigned slots = (unsigned)__cvta_generic_to_shared(sm + (CL ? L.sl : 0));
   typedef typename std::conditional<VG, unsigned, int2>::type Word;
   Word* const win = reinterpret_cast<Word*>(sm + L.wi);
   const int llc = kResSlots * L.llw, llr = llc * S.tiles_x;  // words of a tile, of a row of tiles
@@ -366,7 +387,12 @@ __global__ void __launch_bounds__(res_threads(N, LPE, ADJ), 1)
         else { r = 0; cc = 0; to = L.ll_c; dx = dz = -1; }
         const int wp = (((r / N) / ezc) * sw + (cc / N + 1) * LPE + (r % N) / NJ) >> 5;
         const int at = atomicAdd(&s_wo[pass ? wp : wp + 1], 1);
-        if (pass) word_out(wout[at], to, o0 + r * L.Wp + cc, dx, dz, llc, llr);
+        if (pass) {
+          if constexpr (CL)  // the receiver's rank and the place
+            wout[at] = make_int2(to | (lt + dx + dz * S.tiles_x) << 16, o0 + r * L.Wp + cc);
+          else
+            word_out(wout[at], to, o0 + r * L.Wp + cc, dx, dz, llc, llr);
+        }
       }
       __syncthreads();
       if (pass == 0 && tid == 0)
@@ -506,6 +532,7 @@ __global__ void __launch_bounds__(res_threads(N, LPE, ADJ), 1)
     fetch_w(t_hi - 1);
   }
   __syncthreads();
+  if constexpr (CL) cluster_barrier();  // every CTA's slots are cleared before the first word is sent
 
   const bool fin = !ADJ && kind == RES_FWD && shift;  // one more read-out after the last step
   const int nst = t_hi - t_lo;                        // steps
@@ -529,7 +556,8 @@ __global__ void __launch_bounds__(res_threads(N, LPE, ADJ), 1)
         bool ok = true;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (j == 0 || w0 + j * T < n_in) v[j] = ll_load(in0 + so + word_from(e[j]));
+          if (j == 0 || w0 + j * T < n_in)
+            v[j] = CL ? ll_load_shared(slots + 8u * (unsigned)(so + word_from(e[j]))) : ll_load(in0 + so + word_from(e[j]));
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           if (j == 0 || w0 + j * T < n_in) ok &= (unsigned)(v[j] >> 32) == tag;
@@ -971,9 +999,16 @@ __global__ void __launch_bounds__(res_threads(N, LPE, ADJ), 1)
         for (int j = 0; j < 4; ++j) e[j] = wout[min(w0 + 32 * j, w_hi - 1)];
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[j] = f[word_reg(e[j])];
+        if constexpr (CL) {
+          const unsigned q = slots + 8u * ((tag & (kResSlots - 1)) * (unsigned)L.llw);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)  // (past the end: the last word again)
-          ll_send(p + word_to(e[j], llc, llr), v[j], tag);
+          for (int j = 0; j < 4; ++j)
+            ll_send_cluster(q + 8u * (unsigned)(word_from(e[j]) & 0xffff), word_from(e[j]) >> 16, v[j], tag);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)  // (past the end: the last word again)
+            ll_send(p + word_to(e[j], llc, llr), v[j], tag);
+        }
       }
     }
     // ---- now and then: v at a checkpoint, the gradient's partial sums into the float64 field (while
@@ -998,6 +1033,7 @@ __global__ void __launch_bounds__(res_threads(N, LPE, ADJ), 1)
       }
     }
   }
+  if constexpr (CL) cluster_barrier();  // no CTA leaves while a neighbour may still write to its slots
   if (misfit_on && my_rec && n_fail < 0) {
     S.misfit[my_r] = mis;
     S.rmax[my_r] = rmx;

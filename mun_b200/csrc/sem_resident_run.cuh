@@ -5,25 +5,33 @@ namespace {
 
 SolveIo solve_io(const sem_solve_t& s, const Workspace& ws, char* a);
 
+constexpr int kResSmem = 231424;  // dynamic shared bytes: one CTA per SM, 1 KB left for its static ones
 typedef void (*ResFn)(const SolveDev*, const int*, ResLay, unsigned long long*, unsigned, int, int, int, int, int);
 
 // variants: one lane per element, two (order 4), one with the increment and the partial gradient in
 // memory (adjoint, for meshes whose tiles fit in no other way: 400x200 alone, forward + adjoint, 15.7 us
 // a step, 27.7 by strips; not above order 4, where its registers spill: order 5, 240x150, 26.0 us, 24.2
-// by strips)
-enum : int { RES_ONE = 1, RES_TWO = 2, RES_MEM = 3 };
-int res_lanes(int vr) { return vr == RES_TWO ? 2 : 1; }
-bool res_has(int N, int vr, bool adj) { return vr == RES_ONE || (vr == RES_TWO && N == 4) || (vr == RES_MEM && adj && N <= 4); }
+// by strips); and the first two with each solve's tiles in one cluster
+enum : int { RES_ONE = 1, RES_TWO = 2, RES_MEM = 3, RES_CONE = 4, RES_CTWO = 5, RES_LAST = 5 };
+bool res_clus(int vr) { return vr >= RES_CONE; }
+bool res_two(int vr) { return vr == RES_TWO || vr == RES_CTWO; }
+int res_lanes(int vr) { return res_two(vr) ? 2 : 1; }
+bool res_has(int N, int vr, bool adj) { return vr == RES_MEM ? adj && N <= 4 : !res_two(vr) || N == 4; }
+// Clusters of `size` CTAs that fill an SM each which the device holds at once (a cluster stays within a
+// GPC); size 1, 2, 4, 8 or 16
+int res_clusters(int device, int size);
 
 template <int N, bool ADJ, bool STC>
 ResFn res_fn(int vr) {
   if constexpr (N == 4) {
-    if (vr == RES_TWO) return sem_resident_kernel<N, 2, ADJ, STC, false>;
+    if (vr == RES_TWO) return sem_resident_kernel<N, 2, ADJ, STC, false, false>;
+    if (vr == RES_CTWO) return sem_resident_kernel<N, 2, ADJ, STC, false, true>;
   }
   if constexpr (ADJ && N <= 4) {
-    if (vr == RES_MEM) return sem_resident_kernel<N, 1, ADJ, STC, true>;
+    if (vr == RES_MEM) return sem_resident_kernel<N, 1, ADJ, STC, true, false>;
   }
-  return sem_resident_kernel<N, 1, ADJ, STC, false>;
+  if (vr == RES_CONE) return sem_resident_kernel<N, 1, ADJ, STC, false, true>;
+  return sem_resident_kernel<N, 1, ADJ, STC, false, false>;
 }
 template <bool ADJ, bool STC>
 ResFn res_fn(int N, int vr) {
@@ -41,6 +49,33 @@ ResFn res_fn(int N, int vr) {
 ResFn res_kernel_for(int N, int vr, bool adj, bool stc) {
   if (adj) return stc ? res_fn<true, true>(N, vr) : res_fn<true, false>(N, vr);
   return stc ? res_fn<false, true>(N, vr) : res_fn<false, false>(N, vr);
+}
+
+int res_clusters(int device, int size) {
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, int> have;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto it = have.find(std::make_pair(device, size));
+  if (it != have.end()) return it->second;
+  const ResFn fn = res_kernel_for(4, RES_CTWO, true, false);
+  int n = 0;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3((unsigned)size);
+  lc.blockDim = dim3(512);
+  lc.dynamicSmemBytes = kResSmem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)size;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  if (raise_smem_limit((const void*)fn, kResSmem) != cudaSuccess ||
+      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, fn, &lc) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  return have[std::make_pair(device, size)] = n;
 }
 
 // Receiver lists of the balanced tiling ntx x ntz of a plan (tiles from res_start).
@@ -122,7 +157,7 @@ ResLay res_layout(int N, int vr, bool adj, bool stc, int exm, int ezm, int ezl, 
   ResLay L{};
   const int NP = N + 1;
   // rows of lanes spread over the banks: two lanes per element read rows two apart at once
-  auto pitch = [&](int v) { return vr == RES_TWO ? (v + 7) / 16 * 16 + 8 : 4 * ((v + 3) / 4 | 1); };
+  auto pitch = [&](int v) { return res_two(vr) ? (v + 7) / 16 * 16 + 8 : 4 * ((v + 3) / 4 | 1); };
   L.Rm = ezm * N + 1;
   L.Cm = exm * N + 1;
   L.qx = exm + 1;
@@ -155,13 +190,13 @@ ResLay res_layout(int N, int vr, bool adj, bool stc, int exm, int ezm, int ezl, 
     L.im = take(((long long)rows * L.qx + 1) / 2);
   }
   if (stc) { const int bn = 2 * L.Rm + L.Cm; L.be = take(3LL * bn); L.bd = take(2LL * bn); }
-  L.total = (int)round_up(o, 4);
   L.ll_t = L.Rm * N; L.ll_r = L.ll_t + L.Cm * N; L.ll_b = L.ll_r + L.Rm; L.ll_c = L.ll_b + L.Cm;
   L.llw = (int)round_up(L.ll_c + 1, 16);
+  L.sl = res_clus(vr) ? take(2LL * kResSlots * L.llw) : -1;
+  L.total = (int)round_up(o, 4);
   return L;
 }
 
-constexpr int kResSmem = 231424;  // dynamic shared bytes: one CTA per SM, 1 KB left for its static ones
 // Threads of a launch whose largest tile is exm x ezm elements (the lowest ezl high): lanes per
 // tile row, element rows per chunk, compute and receiver threads; exchange words.
 struct ResShape { int sw, ezc, nc, nio, edge; };
@@ -186,12 +221,16 @@ bool res_shape(int N, int vr, bool adj, int exm, int ezm, int ezl, int nrec, Res
 // swaps between them, which decides full SMs (128 of 100x50: 133 us a step, 142 with two).
 // Two or three smaller CTAs per SM, which hide one another's exchange, measured the same or
 // slower (16 of 100x50 with one lane: 18.1 us a step with one, 18.9 with two, 22.5 with three).
+// A cluster's exchange is shorter, but a solve then has 16 SMs at most (a B200 holds 7 clusters of 16, 15
+// of 8): us a step forward / adjoint, all SMs -> one cluster: 20x10 1.67 / 1.87 -> 1.37 / 1.81, 40x20
+// 1.70 / 1.89 -> 1.67 / 2.07, order 3, 40x20 1.79 / 1.99 -> 1.42 / 1.73, order 5, 37x31 3.07 / 4.83 ->
+// 2.75 / 4.52; order 3, 80x40 1.73 / 2.01 -> 2.20 / 2.08.
 double res_step_cost(int N, int vr, bool adj, const ResShape& h) {
   const double NP = N + 1;
   const double el = adj ? 2 * N * (3 * NP * NP + 4 * NP) + 16 * N * N : 2 * N * (2 * NP * NP + 2 * NP) + 10 * N * N;
   const double carry = N * (NP * NP + 3 * NP) + (adj ? N * (NP + 2) : 0);
-  const double fixed = vr == RES_TWO ? 2600.0 : adj ? 2300.0 : 2500.0;
-  const double rate = !adj ? 1.6 : vr == RES_TWO ? 1.7 : vr == RES_ONE ? 1.9 : 2.1;
+  const double fixed = (res_two(vr) ? 2600.0 : adj ? 2300.0 : 2500.0) - (!res_clus(vr) ? 0.0 : res_two(vr) ? (adj ? 380.0 : 900.0) : adj ? 900.0 : 1050.0);
+  const double rate = !adj ? 1.6 : res_two(vr) ? 1.7 : vr == RES_MEM ? 2.1 : 1.9;
   return fixed + 1.2 * h.edge + rate * std::max(1.0, h.nc / 128.0) * (h.ezc * el + carry) / res_lanes(vr);
 }
 bool res_fits(const ResLay& L) {  // (256: the history box; 4096: the place of a packed exchange word)
@@ -246,7 +285,9 @@ ResTiling res_tiling(const sem_plan_s* p, int vr, bool adj, int E, int sms) {
     const int ezm = E / ex;
     if (ezm < 1 || (ex + 2) * res_lanes(vr) > 32) continue;
     const int tz = (p->nelz + ezm - 1) / ezm, ez = (p->nelz + tz - 1) / tz;
+    const int nt = tx * tz;
     if ((long long)tx * tz > sms) continue;
+    if (res_clus(vr) && (nt > 16 || (nt & (nt - 1)) || !res_clusters(p->device, nt))) continue;
     ResShape h;
     if (!res_shape(p->npol, vr, adj, ex, ez, p->nelz / tz, 1, &h)) continue;
     const double c = res_step_cost(p->npol, vr, adj, h);
@@ -312,9 +353,13 @@ ResPack res_pack(const sem_solve_t* sv, const std::vector<int>& idx, const std::
   }
   const bool stc = plans[0]->bnd_n > 0;
   ResPack best;
+  auto rounds = [&](int size, int count) {  // of a wave of clusters
+    const int at_once = size > 0 ? std::max(1, res_clusters(plans[0]->device, size)) : 1;
+    return (double)((count + at_once - 1) / at_once);
+  };
   std::vector<ResTiling> tl(plans.size()), last;
   std::vector<int> first;
-  for (int vr = RES_ONE; vr <= RES_MEM; ++vr) {
+  for (int vr = RES_ONE; vr <= RES_LAST; ++vr) {
     if (!res_has(N, vr, adj)) continue;
     last.clear();
     res_capacities([&](int E) {
@@ -328,7 +373,7 @@ ResPack res_pack(const sem_solve_t* sv, const std::vector<int>& idx, const std::
       last = tl;
       first.clear();
       double cost = 0.0, step = 0.0;
-      int used = 0, nt = 0, exm = 0, ezm = 0, ezl = 0;
+      int used = 0, nt = 0, exm = 0, ezm = 0, ezl = 0, in_wave = 0;
       ResCounts cnt;
       for (int j = 0; j < n; ++j) {
         const ResTiling& t = tl[pl[j]];
@@ -337,26 +382,29 @@ ResPack res_pack(const sem_solve_t* sv, const std::vector<int>& idx, const std::
         ResCounts c = cnt;
         take_max(c, t.n);
         ResShape h;
-        bool fits = j > 0 && used + t.tx * t.tz <= sms;
+        // a wave of clusters has one size of cluster and needs not be resident at once
+        bool fits = j > 0 && (res_clus(vr) ? t.tx * t.tz == used : used + t.tx * t.tz <= sms);
         if (fits) {
           const int x = std::max(ex, exm), z = std::max(ez, ezm);
           fits = res_shape(N, vr, adj, x, z, std::max(el, ezl), adj ? c.ninj : c.nrec, &h) &&
                  res_fits(res_layout(N, vr, adj, stc, x, z, std::max(el, ezl), c));
         }
         if (!fits) {  // the next wave
-          cost += step * nt;
+          cost += step * (res_clus(vr) ? rounds(used, in_wave) * nt : nt);
+          in_wave = 0;
           first.push_back(j);
           used = nt = exm = ezm = ezl = 0;
           c = t.n;
           res_shape(N, vr, adj, ex, ez, el, adj ? c.ninj : c.nrec, &h);
         }
         cnt = c;
-        used += t.tx * t.tz;
+        used = res_clus(vr) ? t.tx * t.tz : used + t.tx * t.tz;
+        ++in_wave;
         exm = std::max(exm, ex); ezm = std::max(ezm, ez); ezl = std::max(ezl, el);
         step = res_step_cost(N, vr, adj, h);
         nt = std::max(nt, steps[j]);
       }
-      cost += step * nt;
+      cost += step * (res_clus(vr) ? rounds(used, in_wave) * nt : nt);
       if (best.cost >= 0.0 && cost >= best.cost) return;
       best.cost = cost;
       best.vr = vr;
@@ -431,6 +479,7 @@ struct ResWave {
   ResLay L;
   ResShape h;
   int ncta, cta0;           // CTAs, and where their list starts
+  int cluster;              // CTAs per cluster, or 0: a cooperative launch
   const std::vector<int>* solves;
 };
 
@@ -473,14 +522,16 @@ int run_res_group(sem_batch_t* b, const sem_solve_t* sv, char* const* at, const 
       v.L = res_layout(N, pk.vr, q, stc, exm, ezm, ezl, c);
       v.fn = res_kernel_for(N, pk.vr, q, stc);
       if (!res_shape(N, pk.vr, q, exm, ezm, ezl, q ? c.ninj : c.nrec, &v.h)) return SEM_ERR_UNSUPPORTED;
+      v.cluster = res_clus(pk.vr) ? pk.tiles[wv[0]].tx * pk.tiles[wv[0]].tz : 0;
       int nb = 0;
       if (!res_fits(v.L) || raise_smem_limit((const void*)v.fn, (size_t)v.L.total * 4) != cudaSuccess ||
+          (v.cluster > 8 && cudaFuncSetAttribute(v.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, v.fn, v.h.nc + v.h.nio, (size_t)v.L.total * 4) != cudaSuccess ||
-          (long long)nb * sms < v.ncta) {
+          (long long)nb * sms < (v.cluster ? v.cluster : v.ncta)) {
         cudaGetLastError();
         return SEM_ERR_UNSUPPORTED;
       }
-      ll_words = std::max(ll_words, (long long)v.ncta * kResSlots * v.L.llw);
+      if (!v.cluster) ll_words = std::max(ll_words, (long long)v.ncta * kResSlots * v.L.llw);
       if (q)
         for (int j : wv) wave_of[j] = (int)waves[q].size();
       else { b->last_tile_ex = exm; b->last_tile_ez = ezm; }
@@ -638,7 +689,7 @@ int run_res_group(sem_batch_t* b, const sem_solve_t* sv, char* const* at, const 
       }
       if (steps == 0) continue;
       if (b->ll_tag > 0xf0000000u - (unsigned)steps) {
-        CUDA_TRY(cudaMemsetAsync(b->d_ll, 0, b->ll_cap, stream));
+        if (b->d_ll) CUDA_TRY(cudaMemsetAsync(b->d_ll, 0, b->ll_cap, stream));
         b->ll_tag = 0;
       }
       cudaLaunchConfig_t lc = {};
@@ -647,8 +698,14 @@ int run_res_group(sem_batch_t* b, const sem_solve_t* sv, char* const* at, const 
       lc.dynamicSmemBytes = (size_t)v.L.total * 4;
       lc.stream = stream;
       cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeCooperative;
-      at[0].val.cooperative = 1;
+      if (v.cluster) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)v.cluster;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+      }
       lc.attrs = at;
       lc.numAttrs = 1;
       CUDA_TRY(cudaLaunchKernelEx(&lc, v.fn, (const SolveDev*)b->d_solves, (const int*)b->d_cta + v.cta0, v.L, b->d_ll,

@@ -126,3 +126,13 @@ def test_adjoint_tiles_with_fields_in_memory(npol, nelx, nelz, boundary):
     p, c = _plan(nelx, nelz, npol, 120, 8, boundary, circle=True)
     b = _compare(lambda: [_spec(p, c, 3, "gradient")])
     assert b.last_kernel == "resident"
+
+
+@pytest.mark.parametrize("npol,nelx,nelz,models,boundary", [
+    (4, 4, 4, 3, "sponge"), (4, 17, 5, 21, "sponge"), (3, 40, 20, 16, "stacey"), (5, 37, 31, 9, "sponge"),
+    (2, 9, 33, 40, "sponge"), (7, 8, 8, 5, "stacey")])
+def test_solves_as_clusters(npol, nelx, nelz, models, boundary):
+    # a solve per thread-block cluster, alone and with more clusters than the GPU holds at once
+    p, c = _plan(nelx, nelz, npol, 90, 9, boundary, circle=nelx > 8)
+    _compare(lambda: [_spec(p, c, 4, "gradient", ckpt_k=31)])
+    _compare(lambda: [_spec(p, c, 5 + i, "gradient" if i % 3 else "likelihood") for i in range(models)])
