@@ -2092,6 +2092,7 @@ struct sem_plan_s {
   mutable std::map<std::pair<int, int>, ResLists> res_lists;
   struct ResCounts { int nrec = 0, ninj = 0, nquad = 0, nterm = 0; };  // bounds over a tiling's tiles
   struct ResTiling { int tx = 0, tz = 0; ResCounts n; };
+  mutable std::map<std::pair<int, int>, ResCounts> res_tile_counts;     // by tiles in x and z
   mutable int res_need[2] = {-1, -1};  // variants its solves need (forward, adjoint), when known
   mutable std::map<std::tuple<int, bool, int>, ResTiling> res_tilings;  // by variant, adjoint, capacity
   mutable std::mutex mu;

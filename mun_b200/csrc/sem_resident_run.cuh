@@ -222,9 +222,9 @@ bool res_shape(int N, int vr, bool adj, int exm, int ezm, int ezl, int nrec, Res
 // Two or three smaller CTAs per SM, which hide one another's exchange, measured the same or
 // slower (16 of 100x50 with one lane: 18.1 us a step with one, 18.9 with two, 22.5 with three).
 // A cluster's exchange is shorter, but a solve then has 16 SMs at most (a B200 holds 7 clusters of 16, 15
-// of 8): us a step forward / adjoint, all SMs -> one cluster: 20x10 1.67 / 1.87 -> 1.37 / 1.81, 40x20
-// 1.70 / 1.89 -> 1.67 / 2.07, order 3, 40x20 1.79 / 1.99 -> 1.42 / 1.73, order 5, 37x31 3.07 / 4.83 ->
-// 2.75 / 4.52; order 3, 80x40 1.73 / 2.01 -> 2.20 / 2.08.
+// of 8): us a step forward / adjoint, all SMs -> one cluster: 20x10 1.62 / 1.88 -> 1.18 / 1.70, 48x28 forward
+// 1.68 -> 1.51, order 3, 40x20 1.80 / 2.02 -> 1.27 / 1.58, order 5, 37x31 2.95 / 4.85 -> 2.43 / 4.23; with too
+// much work per SM, order 3, 80x40: 1.73 / 2.01 -> 2.20 / 2.08 (before the cluster kernels were compiled apart).
 double res_step_cost(int N, int vr, bool adj, const ResShape& h) {
   const double NP = N + 1;
   const double el = adj ? 2 * N * (3 * NP * NP + 4 * NP) + 16 * N * N : 2 * N * (2 * NP * NP + 2 * NP) + 10 * N * N;
@@ -292,7 +292,11 @@ ResTiling res_tiling(const sem_plan_s* p, int vr, bool adj, int E, int sms) {
     if (!res_shape(p->npol, vr, adj, ex, ez, p->nelz / tz, 1, &h)) continue;
     const double c = res_step_cost(p->npol, vr, adj, h);
     if (best_c >= 0.0 && tx * tz * c >= best_c) continue;
-    const ResCounts cnt = res_counts(p, tx, tz);
+    // (counted once per tiling: the search meets each many times, and a plan may serve one call only)
+    const auto at = p->res_tile_counts.find(std::make_pair(tx, tz));
+    const ResCounts cnt = at != p->res_tile_counts.end()
+                              ? at->second
+                              : (p->res_tile_counts[std::make_pair(tx, tz)] = res_counts(p, tx, tz));
     if (!res_shape(p->npol, vr, adj, ex, ez, p->nelz / tz, adj ? cnt.ninj : cnt.nrec, &h) ||
         !res_fits(res_layout(p->npol, vr, adj, stc, ex, ez, p->nelz / tz, cnt)))
       continue;
