@@ -2466,6 +2466,7 @@ struct sem_batch_s {
   unsigned long long* d_ll = nullptr;   // resident kernels: exchange words, and the last step tag
   long long ll_cap = 0;                 //   used (tags only grow, so stale words never match)
   unsigned ll_tag = 0;
+  bool ll_recorded = false;             //   a captured run's launches may be replayed, with their tags
   char* d_sync = nullptr;               // persistent strip kernel: per-CTA tick counters and
   long long sync_cap = 0;               //   per-solve barrier counters
 };

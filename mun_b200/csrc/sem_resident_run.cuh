@@ -665,6 +665,12 @@ int run_res_group(sem_batch_t* b, const sem_solve_t* sv, char* const* at, const 
     CUDA_TRY(cudaMemsetAsync(b->d_ll, 0, ll_bytes, stream));
     b->ll_tag = 0;
   }
+  // The launches of a captured run carry the same tags at every replay.  So the words are cleared before
+  // them, and, since a replay leaves such tags behind at any time, before all later runs of this batch.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CUDA_TRY(cudaStreamIsCapturing(stream, &cap));
+  b->ll_recorded |= cap != cudaStreamCaptureStatusNone;
+  if (b->ll_recorded && ll_bytes > 0) CUDA_TRY(cudaMemsetAsync(b->d_ll, 0, ll_bytes, stream));
   CUDA_TRY(cudaMemcpyAsync(b->d_solves, b->h_solves.data(), sizeof(SolveDev) * n * nq, cudaMemcpyHostToDevice, stream));
   if (adj)
     CUDA_TRY(cudaMemcpyAsync(b->d_tmaps, b->h_tmaps.data(), sizeof(CUtensorMap) * n, cudaMemcpyHostToDevice, stream));

@@ -1,0 +1,37 @@
+"""Calls that the resident kernels take over from the tick kernels: what callers could do with
+those, they can do with these."""
+import pytest
+import torch
+
+from mun_b200 import Batch
+from tests.test_gpu_resident import _plan, _same, _spec
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape,nt,mode", [((20, 10), 60, "gradient"), ((60, 30), 90, "gradient"), ((60, 30), 91, "forward")])
+def test_captured_run_replays_with_new_inputs(shape, nt, mode):
+    # a captured run is replayed with new velocities; runs of the same batch come between
+    p, c = _plan(*shape, 4, nt, 9, circle=True)
+    kw = {"ckpt_k": 25} if mode == "gradient" else {}
+    s = _spec(p, c, 1, mode, **kw)
+    b, stream, graph = Batch(kernel=5), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        b.run([s])
+    stream.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        b.run([s])
+    first = s.velocity.clone()
+    for scale in (1.0, 0.9, 1.02, 0.97, 1.0):
+        s.velocity.copy_(first * scale)
+        ref = _spec(p, c, 1, mode, **kw)
+        ref.velocity = first * scale
+        Batch(kernel=1).run([ref])
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert b.last_kernel == "resident"
+        _same([ref], [s])
+        b.run([s])
+        torch.cuda.synchronize()
+        _same([ref], [s])
