@@ -191,6 +191,13 @@ int sem_forward_adjoint(sem_batch_t* batch, const sem_plan_t* plan, const double
  * kernel's tick barrier); 2: a grid barrier that completes.  Blocks about 2 s for
  * 0 and 1; *status_out = SEM_ERR_TIMEOUT for 0 and 1, SEM_OK for 2. */
 int sem_selftest_wait(int32_t which, int32_t* status_out);
+/* Host only: the receivers, injected receivers, quads of nodes and terms of the fullest tile
+ * of a resident tiling (tiles_x x tiles_z balanced tiles), as counted when the tiling is
+ * chosen and as found in the lists that it runs with.  rec_base: (x, z) node of each
+ * receiver's element; counted, listed: 4 each. */
+int sem_selftest_receivers(int32_t npol, int32_t nelx, int32_t nelz, int32_t nrec,
+                           const int32_t* rec_base, int32_t tiles_x, int32_t tiles_z,
+                           int32_t* counted, int32_t* listed);
 
 /* Allocation-free forward solve (receivers in the run() convention), for callers that
  * cannot allocate device memory while they run: a caller inside a memory pool that owns

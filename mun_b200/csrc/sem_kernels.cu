@@ -2090,7 +2090,14 @@ struct sem_plan_s {
     int nrec, ninj, nquad, nterm;
   };
   mutable std::map<std::pair<int, int>, ResLists> res_lists;
-  struct ResCounts { int nrec = 0, ninj = 0, nquad = 0, nterm = 0; };  // bounds over a tiling's tiles
+  struct ResCounts { int nrec = 0, ninj = 0, nquad = 0, nterm = 0; };  // most in any tile of a tiling
+  struct ResSites {  // elements with receivers, and the cells of nodes that they reach
+    struct El { int ex, ez, n; };
+    struct Cell { int ex, ez, quads, terms; };
+    std::vector<El> el;
+    std::vector<Cell> cells;
+  };
+  mutable ResSites res_sites;
   struct ResTiling { int tx = 0, tz = 0; ResCounts n; };
   mutable std::map<std::pair<int, int>, ResCounts> res_tile_counts;     // by tiles in x and z
   mutable int res_need[2] = {-1, -1};  // variants its solves need (forward, adjoint), when known
@@ -3260,6 +3267,27 @@ int sem_selftest_wait(int32_t which, int32_t* status_out) {
   cudaFree(buf);
   *status_out = h;
   return rc;
+}
+
+int sem_selftest_receivers(int32_t npol, int32_t nelx, int32_t nelz, int32_t nrec, const int32_t* rec_base,
+                           int32_t tiles_x, int32_t tiles_z, int32_t* counted, int32_t* listed) {
+  if (!counted || !listed || (nrec && !rec_base) || npol < 1 || npol > kMaxN || nrec < 0 || tiles_x < 1 || tiles_z < 1 ||
+      tiles_x > nelx || tiles_z > nelz)
+    return fail(SEM_ERR_ARG, "bad mesh, tiling or receivers");
+  for (int r = 0; r < nrec; ++r)
+    for (int q = 0; q < 2; ++q) {
+      const int at = rec_base[2 * r + q];
+      if (at < 0 || at % npol || at / npol >= (q ? nelz : nelx)) return fail(SEM_ERR_ARG, "receiver outside the mesh");
+    }
+  const ResCounts c = res_counts(res_sites(npol, nrec, rec_base), nelx, nelz, tiles_x, tiles_z);
+  ResListsHost h;
+  build_res_lists(npol, nelx, nelz, nrec, rec_base, nullptr, tiles_x, tiles_z, &h);
+  const ResCounts* const n[2] = {&c, &h.n};
+  int32_t* const out[2] = {counted, listed};
+  for (int q = 0; q < 2; ++q) {
+    out[q][0] = n[q]->nrec; out[q][1] = n[q]->ninj; out[q][2] = n[q]->nquad; out[q][3] = n[q]->nterm;
+  }
+  return SEM_OK;
 }
 
 int sem_forward_noalloc(const sem_plan_t* p, const double* velocity, float* rec_out,

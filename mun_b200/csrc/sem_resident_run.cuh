@@ -78,76 +78,88 @@ int res_clusters(int device, int size) {
   return have[std::make_pair(device, size)] = n;
 }
 
-// Receiver lists of the balanced tiling ntx x ntz of a plan (tiles from res_start).
+typedef sem_plan_s::ResCounts ResCounts;
+typedef sem_plan_s::ResTiling ResTiling;
+typedef sem_plan_s::ResSites ResSites;
+// Tile of element e among n tiles of nel elements: the inverse of res_start (the last one for the
+// mesh's last node).
+int res_owner(int e, int nel, int n) { return e >= nel ? n - 1 : (int)(((long long)e * n) / nel); }
+
+// Receiver lists of the balanced tiling ntx x ntz of a mesh.
+struct ResListsHost {
+  std::vector<int> ro{0}, ri, io{0}, ii, qo{0}, qp, eo, et;
+  std::vector<float> ew;
+  ResCounts n;
+};
+void build_res_lists(int N, int nelx, int nelz, int nrec, const int* base, const float* wts, int ntx, int ntz,
+                     ResListsHost* out) {
+  const int NP = N + 1, nt = ntx * ntz;
+  ResListsHost& L = *out;
+  std::vector<std::vector<int>> rec(nt), inj(nt);
+  // per tile and quad (row << 16 | element): the receivers that reach it, with node masks and weights
+  struct Term { int q, mask; std::vector<float> w; };
+  std::vector<std::map<int, std::vector<Term>>> quads(nt);
+  for (int r = 0; r < nrec; ++r) {
+    const int bx = base[2 * r], bz = base[2 * r + 1];
+    rec[res_owner(bz / N, nelz, ntz) * ntx + res_owner(bx / N, nelx, ntx)].push_back(r);
+    for (int j = 0; j < NP; ++j)
+      for (int i = 0; i < NP; ++i) {
+        const int gx = bx + i, gz = bz + j;
+        const int tx = res_owner(gx / N, nelx, ntx), tz = res_owner(gz / N, nelz, ntz);
+        const int t = tz * ntx + tx;
+        if (inj[t].empty() || inj[t].back() != r) inj[t].push_back(r);
+        const int q = (int)inj[t].size() - 1;
+        const int x0 = res_start(tx, nelx, ntx) * N, z0 = res_start(tz, nelz, ntz) * N;
+        auto& terms = quads[t][((gz - z0) << 16) | ((gx - x0) / N)];
+        if (terms.empty() || terms.back().q != q) terms.push_back(Term{q, 0, std::vector<float>(N, 0.f)});
+        terms.back().mask |= 1 << ((gx - x0) % N);
+        terms.back().w[(gx - x0) % N] = wts ? wts[(size_t)r * NP * NP + j * NP + i] : 0.f;
+      }
+  }
+  for (int t = 0; t < nt; ++t) {
+    L.ri.insert(L.ri.end(), rec[t].begin(), rec[t].end());
+    L.ro.push_back((int)L.ri.size());
+    L.ii.insert(L.ii.end(), inj[t].begin(), inj[t].end());
+    L.io.push_back((int)L.ii.size());
+    const size_t e0 = L.et.size();
+    for (auto& kv : quads[t]) {
+      L.qp.push_back(kv.first);
+      L.eo.push_back((int)L.et.size());
+      for (auto& term : kv.second) {
+        L.et.push_back(term.q << 8 | term.mask);
+        L.ew.insert(L.ew.end(), term.w.begin(), term.w.end());
+      }
+    }
+    L.qo.push_back((int)L.qp.size());
+    L.n.nrec = std::max(L.n.nrec, (int)rec[t].size());
+    L.n.ninj = std::max(L.n.ninj, (int)inj[t].size());
+    L.n.nquad = std::max(L.n.nquad, (int)quads[t].size());
+    L.n.nterm = std::max(L.n.nterm, (int)(L.et.size() - e0));
+  }
+  L.eo.push_back((int)L.et.size());
+}
+// the same on the device, kept with the plan
 int get_res_lists(const sem_plan_s* p, int ntx, int ntz, sem_plan_s::ResLists* out) {
   std::lock_guard<std::mutex> lk(p->mu);
   auto key = std::make_pair(ntx, ntz);
   auto it = p->res_lists.find(key);
   if (it != p->res_lists.end()) { *out = it->second; return SEM_OK; }
-  const int N = p->npol, NP = N + 1;
-  auto owner = [](int e, int nel, int n) {  // tile of element e (the last one for the mesh's last node)
-    return e >= nel ? n - 1 : (int)(((long long)e * n) / nel);
-  };
-  const int nt = ntx * ntz;
-  std::vector<std::vector<int>> rec(nt), inj(nt);
-  // per tile and quad (row << 16 | element): the receivers that reach it, with node masks and weights
-  struct Term { int q, mask; std::vector<float> w; };
-  std::vector<std::map<int, std::vector<Term>>> quads(nt);
-  for (int r = 0; r < p->nrec; ++r) {
-    const int bx = p->h_rec_base[2 * r], bz = p->h_rec_base[2 * r + 1];
-    rec[owner(bz / N, p->nelz, ntz) * ntx + owner(bx / N, p->nelx, ntx)].push_back(r);
-    for (int j = 0; j < NP; ++j)
-      for (int i = 0; i < NP; ++i) {
-        const int gx = bx + i, gz = bz + j;
-        const int tx = owner(gx / N, p->nelx, ntx), tz = owner(gz / N, p->nelz, ntz);
-        const int t = tz * ntx + tx;
-        if (inj[t].empty() || inj[t].back() != r) inj[t].push_back(r);
-        const int q = (int)inj[t].size() - 1;
-        const int x0 = res_start(tx, p->nelx, ntx) * N, z0 = res_start(tz, p->nelz, ntz) * N;
-        auto& terms = quads[t][((gz - z0) << 16) | ((gx - x0) / N)];
-        if (terms.empty() || terms.back().q != q) terms.push_back(Term{q, 0, std::vector<float>(N, 0.f)});
-        terms.back().mask |= 1 << ((gx - x0) % N);
-        terms.back().w[(gx - x0) % N] = p->h_rec_w[(size_t)r * NP * NP + j * NP + i];
-      }
-  }
+  ResListsHost h;
+  build_res_lists(p->npol, p->nelx, p->nelz, p->nrec, p->h_rec_base.data(), p->h_rec_w.data(), ntx, ntz, &h);
   sem_plan_s::ResLists L{};
-  std::vector<int> ro(1, 0), ri, io(1, 0), ii, qo(1, 0), qp, eo, et;
-  std::vector<float> ew;
-  for (int t = 0; t < nt; ++t) {
-    ri.insert(ri.end(), rec[t].begin(), rec[t].end());
-    ro.push_back((int)ri.size());
-    ii.insert(ii.end(), inj[t].begin(), inj[t].end());
-    io.push_back((int)ii.size());
-    const size_t e0 = et.size();
-    for (auto& kv : quads[t]) {
-      qp.push_back(kv.first);
-      eo.push_back((int)et.size());
-      for (auto& term : kv.second) {
-        et.push_back(term.q << 8 | term.mask);
-        ew.insert(ew.end(), term.w.begin(), term.w.end());
-      }
-    }
-    qo.push_back((int)qp.size());
-    L.nrec = std::max(L.nrec, (int)rec[t].size());
-    L.ninj = std::max(L.ninj, (int)inj[t].size());
-    L.nquad = std::max(L.nquad, (int)quads[t].size());
-    L.nterm = std::max(L.nterm, (int)(et.size() - e0));
-  }
-  eo.push_back((int)et.size());
+  L.nrec = h.n.nrec; L.ninj = h.n.ninj; L.nquad = h.n.nquad; L.nterm = h.n.nterm;
   int rc;
-  if ((rc = upload(&L.l.rec_off, ro.data(), ro.size())) || (rc = upload(&L.l.rec_ids, ri.data(), ri.size())) ||
-      (rc = upload(&L.l.inj_off, io.data(), io.size())) || (rc = upload(&L.l.inj_ids, ii.data(), ii.size())) ||
-      (rc = upload(&L.iq_off, qo.data(), qo.size())) || (rc = upload(&L.iq_pos, qp.data(), qp.size())) ||
-      (rc = upload(&L.iterm_off, eo.data(), eo.size())) || (rc = upload(&L.iterm, et.data(), et.size())) ||
-      (rc = upload(&L.iterm_w, ew.data(), ew.size())))
+  if ((rc = upload(&L.l.rec_off, h.ro.data(), h.ro.size())) || (rc = upload(&L.l.rec_ids, h.ri.data(), h.ri.size())) ||
+      (rc = upload(&L.l.inj_off, h.io.data(), h.io.size())) || (rc = upload(&L.l.inj_ids, h.ii.data(), h.ii.size())) ||
+      (rc = upload(&L.iq_off, h.qo.data(), h.qo.size())) || (rc = upload(&L.iq_pos, h.qp.data(), h.qp.size())) ||
+      (rc = upload(&L.iterm_off, h.eo.data(), h.eo.size())) || (rc = upload(&L.iterm, h.et.data(), h.et.size())) ||
+      (rc = upload(&L.iterm_w, h.ew.data(), h.ew.size())))
     return rc;
   p->res_lists[key] = L;
   *out = L;
   return SEM_OK;
 }
 
-typedef sem_plan_s::ResCounts ResCounts;
-typedef sem_plan_s::ResTiling ResTiling;
 void take_max(ResCounts& a, const ResCounts& b) {
   a.nrec = std::max(a.nrec, b.nrec); a.ninj = std::max(a.ninj, b.ninj);
   a.nquad = std::max(a.nquad, b.nquad); a.nterm = std::max(a.nterm, b.nterm);
@@ -237,35 +249,46 @@ bool res_fits(const ResLay& L) {  // (256: the history box; 4096: the place of a
   return L.Wp <= 256 && L.H <= 256 && L.llw <= 4096 && (long long)L.total * 4 <= kResSmem;
 }
 
-// bounds of the receivers of one tile of a tiling
-ResCounts res_counts(const sem_plan_s* p, int ntx, int ntz) {
-  ResCounts c;
-  const int N = p->npol;
-  std::map<int, std::pair<int, std::vector<int>>> tiles;  // receivers and the quads of their first rows
-  for (int r = 0; r < p->nrec; ++r) {
-    const int ex = p->h_rec_base[2 * r] / N, ez = p->h_rec_base[2 * r + 1] / N;
-    int seen[4], ns = 0;
-    for (int q = 0; q < 4; ++q) {  // an element's last nodes may belong to the next tiles
-      const int x = std::min(ex + (q & 1), p->nelx - 1), z = std::min(ez + (q >> 1), p->nelz - 1);
-      const int tx = std::min((int)(((long long)(x + 1) * ntx - 1) / p->nelx), ntx - 1);
-      const int tz = std::min((int)(((long long)(z + 1) * ntz - 1) / p->nelz), ntz - 1);
-      const int t = tz * ntx + tx;
-      if (std::find(seen, seen + ns, t) != seen + ns) continue;
-      seen[ns++] = t;
-      auto& e = tiles[t];
-      e.first++;
-      for (int i = 0; i < 2; ++i) {
-        const int quad = ez * (p->nelx + 1) + ex + i;
-        if (std::find(e.second.begin(), e.second.end(), quad) == e.second.end()) e.second.push_back(quad);
-      }
+// Where a mesh's receivers are, whatever the tiling: elements with receivers, and the cells (one
+// element's own columns of nodes times one element row's own rows) that they reach, with their quads
+// (rows of N nodes) and the receivers' terms in them.  The last row and column of an element's nodes
+// are the next cells'.
+ResSites res_sites(int N, int nrec, const int* base) {
+  std::map<std::pair<int, int>, int> el;                     // receivers by element (z, x)
+  std::map<std::pair<int, int>, std::pair<int, int>> cells;  // quads and terms by cell (z, x)
+  for (int r = 0; r < nrec; ++r) ++el[std::make_pair(base[2 * r + 1] / N, base[2 * r] / N)];
+  for (auto& kv : el)
+    for (int q = 0; q < 4; ++q) {
+      const int rows = q < 2 ? N : 1;
+      auto& c = cells[std::make_pair(kv.first.first + (q >> 1), kv.first.second + (q & 1))];
+      c.first = std::max(c.first, rows);
+      c.second += rows * kv.second;
     }
+  ResSites s;
+  for (auto& kv : el) s.el.push_back({kv.first.second, kv.first.first, kv.second});
+  for (auto& kv : cells) s.cells.push_back({kv.first.second, kv.first.first, kv.second.first, kv.second.second});
+  return s;
+}
+// The largest counts that build_res_lists finds in any tile of a tiling, without the lists: a search
+// meets many tilings, and a mesh may have thousands of receivers (first forward call of a plan, 100x50
+// with 8000: 40 ms when each tiling went through all receivers, 11 now; 60x30 with 5000: 25 and 6.5).
+ResCounts res_counts(const ResSites& s, int nelx, int nelz, int ntx, int ntz) {
+  std::vector<int> ox(nelx + 1), oz(nelz + 1);
+  for (int e = 0; e <= nelx; ++e) ox[e] = res_owner(e, nelx, ntx);
+  for (int e = 0; e <= nelz; ++e) oz[e] = res_owner(e, nelz, ntz) * ntx;
+  std::vector<ResCounts> t((size_t)ntx * ntz);
+  ResCounts c;
+  for (const auto& e : s.el) {
+    t[oz[e.ez] + ox[e.ex]].nrec += e.n;
+    for (int z = 0; z < (oz[e.ez + 1] != oz[e.ez] ? 2 : 1); ++z)
+      for (int x = 0; x < (ox[e.ex + 1] != ox[e.ex] ? 2 : 1); ++x) t[oz[e.ez + z] + ox[e.ex + x]].ninj += e.n;
   }
-  for (auto& kv : tiles) {
-    c.nrec = std::max(c.nrec, kv.second.first);
-    c.nquad = std::max(c.nquad, (int)kv.second.second.size() * (N + 1));
+  for (const auto& e : s.cells) {
+    ResCounts& q = t[oz[e.ez] + ox[e.ex]];
+    q.nquad += e.quads;
+    q.nterm += e.terms;
   }
-  c.ninj = c.nrec;
-  c.nterm = c.ninj * 2 * (N + 1);
+  for (const ResCounts& q : t) take_max(c, q);
   return c;
 }
 
@@ -276,6 +299,7 @@ ResTiling res_tiling(const sem_plan_s* p, int vr, bool adj, int E, int sms) {
   const auto key = std::make_tuple(vr, adj, E);
   auto it = p->res_tilings.find(key);
   if (it != p->res_tilings.end()) return it->second;
+  if (p->nrec > 0 && p->res_sites.el.empty()) p->res_sites = res_sites(p->npol, p->nrec, p->h_rec_base.data());
   ResTiling best;
   double best_c = -1.0;
   const bool stc = p->bnd_n > 0;
@@ -296,7 +320,7 @@ ResTiling res_tiling(const sem_plan_s* p, int vr, bool adj, int E, int sms) {
     const auto at = p->res_tile_counts.find(std::make_pair(tx, tz));
     const ResCounts cnt = at != p->res_tile_counts.end()
                               ? at->second
-                              : (p->res_tile_counts[std::make_pair(tx, tz)] = res_counts(p, tx, tz));
+                              : (p->res_tile_counts[std::make_pair(tx, tz)] = res_counts(p->res_sites, p->nelx, p->nelz, tx, tz));
     if (!res_shape(p->npol, vr, adj, ex, ez, p->nelz / tz, adj ? cnt.ninj : cnt.nrec, &h) ||
         !res_fits(res_layout(p->npol, vr, adj, stc, ex, ez, p->nelz / tz, cnt)))
       continue;

@@ -1,9 +1,10 @@
 """Calls that the resident kernels take over from the tick kernels: what callers could do with
 those, they can do with these."""
+import numpy as np
 import pytest
 import torch
 
-from mun_b200 import Batch
+from mun_b200 import Batch, SEMPlan
 from tests.test_gpu_resident import _plan, _same, _spec
 
 pytestmark = pytest.mark.gpu
@@ -35,3 +36,17 @@ def test_captured_run_replays_with_new_inputs(shape, nt, mode):
         b.run([s])
         torch.cuda.synchronize()
         _same([ref], [s])
+
+
+def test_dense_array_on_one_side_stays_resident():
+    # most receivers lie in one tile of a tiling that divides the mesh unevenly
+    p, c = _plan(56, 31, 5, 60, 1)
+    p = SEMPlan(**dict(p.kwargs, receivers=np.array([(181.0 + 0.2 * i, 61.0 + 1.7 * i) for i in range(81)])))
+    ref, got = ([_spec(p, c, 20 + i, "gradient") for i in range(16)] for _ in range(2))
+    Batch(kernel=1).run(ref)
+    b = Batch(kernel=5)
+    b.run(got)
+    torch.cuda.synchronize()
+    assert b.last_kernel == "resident"
+    for r, s in zip(ref, got):
+        assert torch.equal(r.rec, s.rec) and torch.equal(r.loglik, s.loglik) and torch.equal(r.grad, s.grad)
