@@ -246,6 +246,10 @@ typedef struct {
 
 int sem_engine_create(const sem_engine_cfg_t* cfg, sem_engine_t** out);
 int sem_engine_destroy(sem_engine_t* engine);
+/* Diagnostics: of the groups of solves that the engine's next steps march, `skip` run and the
+ * `count` after them fail with SEM_ERR_OOM before anything of them is launched (as when their
+ * descriptors cannot be allocated). */
+int sem_selftest_fail_marches(sem_engine_t* engine, int32_t skip, int32_t count);
 /* queue one solve (same fields as in sem_run; its buffers must stay valid until it is
  * released) and return a ticket */
 int sem_engine_submit(sem_engine_t* engine, const sem_solve_t* solve, int64_t* ticket);

@@ -57,7 +57,8 @@ EXPORTS = ["sem_plan_create", "sem_plan_destroy", "sem_plan_workspace_bytes", "s
            "sem_batch_destroy", "sem_run", "sem_batch_last_launches", "sem_batch_last_kernel",
            "sem_batch_last_groups", "sem_batch_last_shape", "sem_batch_last_ticks",
            "sem_batch_last_tick_ms", "sem_forward",
-           "sem_forward_adjoint", "sem_forward_noalloc", "sem_selftest_wait", "sem_selftest_receivers", "sem_engine_create", "sem_engine_destroy",
+           "sem_forward_adjoint", "sem_forward_noalloc", "sem_selftest_wait", "sem_selftest_receivers",
+           "sem_selftest_fail_marches", "sem_engine_create", "sem_engine_destroy",
            "sem_engine_submit", "sem_engine_step", "sem_engine_status", "sem_engine_release",
            "sem_engine_stats", "sem_velocity_from_curve", "sem_project_from_curve",
            "sem_velocity_last_error", "sem_last_error"]
@@ -104,6 +105,7 @@ def load(path=None):
     lib.sem_forward_noalloc.argtypes = [vp, vp, vp, vp, vp]
     lib.sem_selftest_wait.argtypes = [i32, vp]
     lib.sem_selftest_receivers.argtypes = [i32, i32, i32, i32, vp, i32, i32, vp, vp]
+    lib.sem_selftest_fail_marches.argtypes = [vp, i32, i32]
     lib.sem_engine_create.argtypes = [C.POINTER(EngineCfg), C.POINTER(vp)]
     lib.sem_engine_destroy.argtypes = [vp]
     lib.sem_engine_submit.argtypes = [vp, C.POINTER(Solve), C.POINTER(i64)]

@@ -81,6 +81,7 @@ int fail(int code, const std::string& msg) {
   do {                                                                           \
     cudaError_t _e = (expr);                                                     \
     if (_e != cudaSuccess) {                                                     \
+      cudaGetLastError(); /* reported here, not again by the next call */        \
       return fail(_e == cudaErrorMemoryAllocation ? SEM_ERR_OOM : SEM_ERR_CUDA,  \
                   std::string(#expr) + ": " + cudaGetErrorString(_e));           \
     }                                                                            \
@@ -2474,6 +2475,7 @@ struct sem_batch_s {
   long long ll_cap = 0;                 //   used (tags only grow, so stale words never match)
   unsigned ll_tag = 0;
   bool ll_recorded = false;             //   a captured run's launches may be replayed, with their tags
+  int fail_skip = 0, fail_groups = 0;   // diagnostics: resident groups that run, then groups that fail
   char* d_sync = nullptr;               // persistent strip kernel: per-CTA tick counters and
   long long sync_cap = 0;               //   per-solve barrier counters
 };
@@ -3542,13 +3544,20 @@ void free_marched(sem_engine_s* e, bool all) {
 }
 
 // Launches the admitted solves that run resident, forward ones first (their results are due first), and
-// leaves the others, in their order, in `admitted`.
+// leaves the others, in their order, in `admitted`; after an error those too that were not launched.
 int engine_march(sem_engine_s* e, std::vector<EngineJob*>* admitted, cudaStream_t stream) {
   if (!e->res)
     if (int rc = sem_batch_create(&e->res)) return rc;
   sem_batch_t* b = e->res;
+  // (the events first: a solve that was launched has one)
+  cudaEvent_t end = nullptr;
+  CUDA_TRY(cudaEventCreateWithFlags(&end, cudaEventDisableTiming));
+  e->marches.push_back(end);
+  for (EngineJob* j : *admitted)
+    if (j->march) CUDA_TRY(cudaEventCreateWithFlags(&j->ev, cudaEventDisableTiming));
   std::vector<char> done(admitted->size(), 0);
-  for (int adj = 0; adj < 2; ++adj) {
+  int rc = SEM_OK;
+  for (int adj = 0; adj < 2 && !rc; ++adj) {
     std::vector<size_t> of;
     std::vector<sem_solve_t> sv;
     std::vector<char*> at;
@@ -3564,30 +3573,44 @@ int engine_march(sem_engine_s* e, std::vector<EngineJob*>* admitted, cudaStream_
     b->last_launches = 0;
     b->tick_ev_used = 0;
     std::vector<int> rest;
+    std::vector<char> ran(of.size(), 0);
     // (no budget: the workspaces are there)
-    if (int rc = run_resident(b, sv.data(), at.data(), (int)sv.size(), LLONG_MAX / 2, stream, &rest)) return rc;
+    rc = run_resident(b, sv.data(), at.data(), (int)sv.size(), LLONG_MAX / 2, stream, &rest, &ran);
     e->launches += b->last_launches;
     for (size_t i = 0; i < of.size(); ++i) {
-      if (std::find(rest.begin(), rest.end(), (int)i) != rest.end()) continue;
+      if (!ran[i]) continue;
       EngineJob* j = (*admitted)[of[i]];
-      CUDA_TRY(cudaEventCreateWithFlags(&j->ev, cudaEventDisableTiming));
-      CUDA_TRY(cudaEventRecord(j->ev, stream));
+      const cudaError_t err = cudaEventRecord(j->ev, stream);
+      if (err != cudaSuccess && !rc) rc = fail(SEM_ERR_CUDA, cudaGetErrorString(err));
       j->state = 2;
       e->marched.push_back(j);
       done[of[i]] = 1;
     }
   }
+  CUDA_TRY(cudaEventRecord(end, stream));
   size_t keep = 0;
-  for (size_t i = 0; i < admitted->size(); ++i)
-    if (!done[i]) (*admitted)[keep++] = (*admitted)[i];
-  if (keep < admitted->size()) {
-    cudaEvent_t ev;
-    CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    e->marches.push_back(ev);
-    CUDA_TRY(cudaEventRecord(ev, stream));
+  for (size_t i = 0; i < admitted->size(); ++i) {
+    EngineJob* j = (*admitted)[i];
+    if (done[i]) continue;
+    if (j->ev) cudaEventDestroy(j->ev);
+    j->ev = nullptr;
+    (*admitted)[keep++] = j;
   }
   admitted->resize(keep);
-  return SEM_OK;
+  return rc;
+}
+
+// admitted solves that were not launched back to the head of the queue
+void engine_unadmit(sem_engine_s* e, const std::vector<EngineJob*>& admitted) {
+  for (size_t i = admitted.size(); i-- > 0;) {
+    EngineJob* j = admitted[i];
+    if (j->ev) cudaEventDestroy(j->ev);
+    j->ev = nullptr;
+    arena_free(e, j->off, j->ws.bytes);
+    j->off = -1;
+    j->state = 0;
+    e->queue.push_front(j);
+  }
 }
 
 }  // namespace
@@ -3698,6 +3721,15 @@ int sem_engine_release(sem_engine_t* e, int64_t ticket) {
   return SEM_OK;
 }
 
+int sem_selftest_fail_marches(sem_engine_t* e, int32_t skip, int32_t count) {
+  if (!e || skip < 0 || count < 0) return fail(SEM_ERR_ARG, "null argument or negative count");
+  if (!e->res)
+    if (int rc = sem_batch_create(&e->res)) return rc;
+  e->res->fail_skip = skip;
+  e->res->fail_groups = count;
+  return SEM_OK;
+}
+
 int sem_engine_stats(const sem_engine_t* e, int64_t* out) {
   if (!e || !out) return fail(SEM_ERR_ARG, "null argument");
   out[0] = (int64_t)e->queue.size();
@@ -3769,7 +3801,10 @@ int sem_engine_step(sem_engine_t* e, void* stream_v) {
   }
   // ---- solves that fit on chip march at once, on the stream behind the outputs above
   if (std::any_of(admitted.begin(), admitted.end(), [](EngineJob* j) { return j->march > 0; }))
-    if (int rc = engine_march(e, &admitted, stream)) return rc;
+    if (int rc = engine_march(e, &admitted, stream)) {
+      engine_unadmit(e, admitted);
+      return rc;
+    }
   // ---- the others run by ticks from here
   const int nadm = (int)admitted.size();
   for (EngineJob* j : admitted) {

@@ -514,6 +514,11 @@ struct ResWave {
 // One group: set-up, forward launches, (replay and) adjoint launches, outputs.  at: the solves'
 // workspaces, or null (the batch's arena).  SEM_ERR_UNSUPPORTED without a message when the group cannot run this way (nothing launched).
 int run_res_group(sem_batch_t* b, const sem_solve_t* sv, char* const* at, const ResGroup& w, int sms, cudaStream_t stream) {
+  if (b->fail_groups > 0 && b->fail_skip-- <= 0) {
+    b->fail_skip = 0;
+    --b->fail_groups;
+    return fail(SEM_ERR_OOM, "resident group refused by sem_selftest_fail_marches");
+  }
   const int n = (int)w.idx.size();
   const sem_plan_s* p0 = sv[w.idx[0]].plan;
   const int N = p0->npol;
@@ -788,9 +793,10 @@ int res_class(const sem_solve_t& s, int sms) {
   return need == RES_MEM && s.ckpt_k > 0 && s.ckpt_k < s.plan->nt ? 0 : need;
 }
 
-// Runs what can run resident and returns the solves that cannot in `rest`.  at: see run_res_group.
+// Runs what can run resident and returns the solves that cannot in `rest`.  at: see run_res_group.  ran:
+// set for the solves that were launched, also when a later group fails.
 int run_resident(sem_batch_t* b, const sem_solve_t* sv, char* const* at, int n, long long budget, cudaStream_t stream,
-                 std::vector<int>* rest) {
+                 std::vector<int>* rest, std::vector<char>* ran = nullptr) {
   const int sms = sm_count(b->device);
   std::map<std::tuple<int, bool, bool, int>, std::vector<int>> classes;
   for (int i = 0; i < n; ++i) {
@@ -807,6 +813,7 @@ int run_resident(sem_batch_t* b, const sem_solve_t* sv, char* const* at, int n, 
       const int rc = run_res_group(b, sv, at, g, sms, stream);
       if (rc == SEM_ERR_UNSUPPORTED) rest->insert(rest->end(), g.idx.begin(), g.idx.end());
       else if (rc) return rc;
+      else if (ran) for (int i : g.idx) (*ran)[i] = 1;
     }
   }
   std::sort(rest->begin(), rest->end());

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from mun_b200 import Batch, SolveSpec
+from mun_b200 import Batch, SolveSpec, _lib
 from mun_b200.serving import Engine, Request, serve
 from tests.goldens import INJECT, load
 from tests.gpu_cases import aligned_obs, dev, plan_for
@@ -110,3 +110,41 @@ def test_engine_marches_beside_ticks():
         assert a.loglik is None or torch.equal(a.loglik, b.loglik)
         assert a.grad is None or torch.equal(a.grad, b.grad)
     assert eng.stats()["bytes_in_use"] == 0 and eng.stats()["running"] == 0
+
+
+@pytest.mark.parametrize("skip", [0, 1, 2])
+def test_failed_march_gives_its_requests_back(skip):
+    # a march's group cannot be set up: the requests of the groups before it are done, the others,
+    # a solve by ticks among them, wait in the queue and finish with the next steps
+    makers = _specs()
+    kinds = [0, 1, 2, 3, 4, 5, 12, 13]  # gradients, likelihoods and forward solves of two orders and more
+    g = load(INJECT[0])
+    long_ = plan_for(g["config"], g["dt"], 20100)
+
+    def make(i):
+        return SolveSpec(long_, dev(np.asarray(g["velocity"]))) if i == 3 else makers[kinds[i]]()
+    alone = [make(i) for i in range(len(kinds))]
+    for s in alone:
+        Batch().run([s])
+    eng = Engine(max_solves=32, memory_cap_bytes=2 << 30, ticks_per_step=64)
+    tickets = [eng.submit(make(i)) for i in range(len(kinds))]
+    _lib.check(eng._lib.sem_selftest_fail_marches(eng.handle, skip, 2))
+    for _ in range(2):
+        before = eng.stats()
+        with pytest.raises(MemoryError):
+            eng.step()
+        torch.cuda.synchronize()
+        done = [t for t in tickets if eng.state(t) == 2]
+        assert all(eng.state(t) == 0 for t in tickets if t not in done)
+        assert len(done) + eng.stats()["queued"] == len(tickets) and before["queued"] >= eng.stats()["queued"]
+        assert (len(done) > 0) == (skip > 0)
+        assert eng.stats()["bytes_in_use"] == 0 and eng.stats()["running"] == 0
+    eng.run_until_done(tickets)
+    torch.cuda.synchronize()
+    for t, a in zip(tickets, alone):
+        b = eng.release(t)
+        assert int(b.status.item()) == 0
+        assert torch.equal(a.rec, b.rec)
+        assert a.loglik is None or torch.equal(a.loglik, b.loglik)
+        assert a.grad is None or torch.equal(a.grad, b.grad)
+    assert eng.stats()["bytes_in_use"] == 0 and eng.stats()["running"] == 0 and eng.stats()["queued"] == 0
