@@ -3172,9 +3172,21 @@ int sem_run(sem_batch_t* b, const sem_solve_t* solves, int32_t n, const sem_laun
     if (int rc = check_solve(b, solves[i])) return rc;
     any_auto |= (solves[i].flags & SEM_F_ADJOINT) && solves[i].ckpt_k <= 0;
   }
-  long long budget = cfg.memory_budget;
   const bool resident = cfg.kernel == 5 || (cfg.kernel == 0 && cfg.graph_chunk <= 0 && cfg.tile_ex == 0 && cfg.strip_bands == 0);
-  if (budget == 0 && (any_auto || resident)) {
+  // memory_budget is for automatic intervals.  A batch without any is split only where it does not fit
+  // the device, and the device is asked (0.09 ms) only when the arena has to grow.
+  long long budget = any_auto ? cfg.memory_budget : LLONG_MAX / 2;
+  bool ask = any_auto && budget == 0;
+  if (!any_auto && resident) {
+    long long total = 0;
+    for (int i = 0; i < n; ++i) {
+      int ns;
+      const bool adj = solves[i].flags & SEM_F_ADJOINT;
+      total += layout(solves[i].plan, solves[i].flags, adj ? std::max(2, std::min(solves[i].ckpt_k, solves[i].plan->nt)) : 2, &ns).bytes;
+    }
+    ask = total > b->arena_bytes;
+  }
+  if (ask) {
     size_t fr = 0, tot = 0;
     CUDA_TRY(cudaMemGetInfo(&fr, &tot));
     budget = (long long)(0.85 * (double)((long long)fr + b->arena_bytes)) - (512LL << 20);

@@ -50,3 +50,18 @@ def test_dense_array_on_one_side_stays_resident():
     assert b.last_kernel == "resident"
     for r, s in zip(ref, got):
         assert torch.equal(r.rec, s.rec) and torch.equal(r.loglik, s.loglik) and torch.equal(r.grad, s.grad)
+
+
+@pytest.mark.parametrize("mode,kw", [("forward", {}), ("likelihood", {}), ("gradient", {"ckpt_k": 20})])
+def test_memory_budget_is_for_automatic_intervals(mode, kw):
+    # a batch without automatic intervals runs as it does without a budget
+    p, c = _plan(20, 10, 4, 50, 7, circle=True)
+    b, seen, ref = Batch(), [], None
+    for budget in (None, 2 * p.workspace_bytes(13 if mode == "gradient" else 0, 20)):
+        got = [_spec(p, c, i, mode, **kw) for i in range(12)]
+        b.run(got, memory_budget=budget)
+        torch.cuda.synchronize()
+        seen.append((b.last_kernel, b.last_groups, b.last_launches))
+        _same(ref or got, got)
+        ref = got
+    assert seen[0] == seen[1] and seen[0][0] == "resident"
