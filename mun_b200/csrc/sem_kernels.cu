@@ -3195,7 +3195,7 @@ int sem_run(sem_batch_t* b, const sem_solve_t* solves, int32_t n, const sem_laun
   std::vector<sem_solve_t> left;
   if (resident) {
     std::vector<int> rest;
-    if (int rc = run_resident(b, solves, nullptr, n, budget, stream, &rest)) return rc;
+    if (int rc = run_resident(b, solves, nullptr, n, budget, cfg.kernel == 5, stream, &rest)) return rc;
     if (rest.empty()) return SEM_OK;
     if (cfg.kernel == 5) cfg.kernel = 0;
     for (int i : rest) left.push_back(solves[i]);
@@ -3587,7 +3587,7 @@ int engine_march(sem_engine_s* e, std::vector<EngineJob*>* admitted, cudaStream_
     std::vector<int> rest;
     std::vector<char> ran(of.size(), 0);
     // (no budget: the workspaces are there)
-    rc = run_resident(b, sv.data(), at.data(), (int)sv.size(), LLONG_MAX / 2, stream, &rest, &ran);
+    rc = run_resident(b, sv.data(), at.data(), (int)sv.size(), LLONG_MAX / 2, false, stream, &rest, &ran);
     e->launches += b->last_launches;
     for (size_t i = 0; i < of.size(); ++i) {
       if (!ran[i]) continue;

@@ -793,9 +793,36 @@ int res_class(const sem_solve_t& s, int sms) {
   return need == RES_MEM && s.ckpt_k > 0 && s.ckpt_k < s.plan->nt ? 0 : need;
 }
 
-// Runs what can run resident and returns the solves that cannot in `rest`.  at: see run_res_group.  ran:
-// set for the solves that were launched, also when a later group fails.
-int run_resident(sem_batch_t* b, const sem_solve_t* sv, char* const* at, int n, long long budget, cudaStream_t stream,
+// Whether a class of solves runs faster by ticks, although it fits the SMs.  Times: 400 steps of solves
+// with 20 m elements, by ticks -> resident.
+bool ticks_win(const sem_solve_t* sv, const std::vector<int>& cls, int sms) {
+  const sem_plan_s* p0 = sv[cls[0]].plan;
+  const bool adj = sv[cls[0]].flags & SEM_F_ADJOINT, stc = p0->bnd_n > 0;
+  long long elements = 0, chunks = 0;
+  for (int i : cls) {
+    const sem_plan_s* p = sv[i].plan;
+    elements += (long long)p->nelx * p->nelz;
+    chunks += (long long)strips_of(p, nullptr) * ((p->nelz + kMinChunk - 1) / kMinChunk);
+  }
+  const double each = (double)elements / cls.size();
+  if (p0->npol == 7) {
+    // A lane's element of order 7 does not fit its registers (500 to 1200 bytes spilled): 6 us a forward
+    // step and 10 an adjoint one, however small the tile.  Where a tick takes its least time too it is
+    // faster: gradients 28x14 6.2 -> 8.0 ms, 23x11 6.4 -> 6.9 (but 11x6 6.6 -> 6.2, 57x29 8.4 -> 8.0, 4 of
+    // 23x11 7.2 -> 6.9); with Stacey edges, gradients 23x11 6.4 -> 8.0, 4 of 16x8 6.7 -> 8.1 (6x3 8.2 -> 7.2,
+    // 4 of 34x17 10.3 -> 8.2), forward 23x11 2.6 -> 2.9, 8 of 11x6 2.6 -> 2.8 (8 of 16x8 3.0 -> 2.7).
+    if (stc ? (adj ? each >= 60 && elements < 2000 : elements < 1000) : adj && each >= 120 && elements < 800) return true;
+    // And strips that fill the GPU hide what one warp waits for: sponge gradients, 2 of 157x79 12.5 -> 18.9,
+    // 16 of 57x29 21.2 -> 23.9 (forward 8.0 -> 6.2; Stacey gradients 64 of 23x11 27.5 -> 19.8).
+    if (adj && !stc && strip_fills(chunks, sms)) return true;
+  }
+  return false;
+}
+
+// Runs what can run resident and returns the solves that cannot in `rest`; unless `all`, those too that
+// are faster by ticks.  at: see run_res_group.  ran: set for the solves that were launched, also when a
+// later group fails.
+int run_resident(sem_batch_t* b, const sem_solve_t* sv, char* const* at, int n, long long budget, bool all, cudaStream_t stream,
                  std::vector<int>* rest, std::vector<char>* ran = nullptr) {
   const int sms = sm_count(b->device);
   std::map<std::tuple<int, bool, bool, int>, std::vector<int>> classes;
@@ -807,6 +834,10 @@ int run_resident(sem_batch_t* b, const sem_solve_t* sv, char* const* at, int n, 
     else classes[std::make_tuple(p->npol, p->bnd_n > 0, adj, need)].push_back(i);
   }
   for (auto& kv : classes) {
+    if (!all && ticks_win(sv, kv.second, sms)) {
+      rest->insert(rest->end(), kv.second.begin(), kv.second.end());
+      continue;
+    }
     const std::vector<ResGroup> groups = res_plan(sv, kv.second, sms, budget);
     if (groups.empty()) { rest->insert(rest->end(), kv.second.begin(), kv.second.end()); continue; }
     for (const ResGroup& g : groups) {

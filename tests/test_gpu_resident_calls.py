@@ -65,3 +65,25 @@ def test_memory_budget_is_for_automatic_intervals(mode, kw):
         _same(ref or got, got)
         ref = got
     assert seen[0] == seen[1] and seen[0][0] == "resident"
+
+
+@pytest.mark.parametrize("npol,shape,nt,models,boundary,mode,kw,kernel", [
+    (7, (23, 11), 40, 1, "sponge", "gradient", {}, "tile"),        # a tick's least time is less than a step's
+    (7, (23, 11), 40, 4, "stacey", "gradient", {}, "tile"),
+    (7, (23, 11), 40, 1, "stacey", "forward", {}, "tile"),
+    (7, (157, 79), 20, 2, "sponge", "gradient", {}, "strip"),      # strips fill the GPU
+    (7, (11, 6), 40, 1, "sponge", "gradient", {}, "resident"),
+    (7, (23, 11), 40, 1, "sponge", "forward", {}, "resident"),
+    (7, (57, 29), 40, 2, "stacey", "gradient", {}, "resident"),
+])
+def test_automatic_kernel_is_the_faster_one(npol, shape, nt, models, boundary, mode, kw, kernel):
+    p, c = _plan(*shape, npol, nt, 9, boundary, circle=shape[0] > 8)
+    ref, got = ([_spec(p, c, 3 + i, mode, **kw) for i in range(models)] for _ in range(2))
+    Batch(kernel=5).run(ref)
+    b = Batch()
+    b.run(got)
+    torch.cuda.synchronize()
+    assert b.last_kernel == kernel
+    for r, s in zip(ref, got):
+        assert int(r.status.item()) == int(s.status.item()) == 0 and torch.equal(r.rec, s.rec)
+        assert r.grad is None or torch.equal(r.grad, s.grad)
