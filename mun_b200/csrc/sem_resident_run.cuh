@@ -798,13 +798,21 @@ int res_class(const sem_solve_t& s, int sms) {
 bool ticks_win(const sem_solve_t* sv, const std::vector<int>& cls, int sms) {
   const sem_plan_s* p0 = sv[cls[0]].plan;
   const bool adj = sv[cls[0]].flags & SEM_F_ADJOINT, stc = p0->bnd_n > 0;
-  long long elements = 0, chunks = 0;
+  long long elements = 0, chunks = 0, points = 0;
+  int nt = 0;
   for (int i : cls) {
     const sem_plan_s* p = sv[i].plan;
+    points += p->npoints;
+    nt = std::max(nt, p->nt);
     elements += (long long)p->nelx * p->nelz;
     chunks += (long long)strips_of(p, nullptr) * ((p->nelz + kMinChunk - 1) / kMinChunk);
   }
   const double each = (double)elements / cls.size();
+  // A march has a prologue (20 us a wave of solves) that few steps do not pay for, the fewer the more waves
+  // there are: forward, one 100x50, 1 step 0.05 -> 0.06 ms (5 steps 0.07, both); 32 of them, 5 steps
+  // 0.25 -> 0.28 (12 steps 0.41 -> 0.35); 128 of them, 12 steps 1.19 -> 1.41 (24 steps 2.0, both); gradients
+  // 0.14 -> 0.18 (0.19, both), 0.67 -> 0.80 (1.10 -> 1.02), 3.2 -> 3.6 (5.3 -> 5.0).
+  if (nt <= 5.0 + 1.2e-6 * (double)points) return true;
   if (p0->npol == 7) {
     // A lane's element of order 7 does not fit its registers (500 to 1200 bytes spilled): 6 us a forward
     // step and 10 an adjoint one, however small the tile.  Where a tick takes its least time too it is

@@ -72,6 +72,10 @@ def test_memory_budget_is_for_automatic_intervals(mode, kw):
     (7, (23, 11), 40, 4, "stacey", "gradient", {}, "tile"),
     (7, (23, 11), 40, 1, "stacey", "forward", {}, "tile"),
     (7, (157, 79), 20, 2, "sponge", "gradient", {}, "strip"),      # strips fill the GPU
+    (4, (20, 10), 5, 1, "sponge", "forward", {}, "tile"),          # few steps
+    (4, (100, 50), 8, 33, "sponge", "gradient", {}, "strip"),
+    (4, (20, 10), 6, 1, "sponge", "forward", {}, "resident"),
+    (4, (100, 50), 9, 33, "sponge", "gradient", {}, "resident"),
     (7, (11, 6), 40, 1, "sponge", "gradient", {}, "resident"),
     (7, (23, 11), 40, 1, "sponge", "forward", {}, "resident"),
     (7, (57, 29), 40, 2, "stacey", "gradient", {}, "resident"),
