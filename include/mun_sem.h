@@ -129,9 +129,10 @@ typedef struct {
                                  auto, with tile, strip_bands and graph_chunk left 0: the
                                  resident kernels for every solve that fits the SMs, but
                                  for kinds of batches where ticks measured faster (some of
-                                 order 7, a few time steps; 5 takes the resident kernels
-                                 there too), and, for the rest, strips when the batch has
-                                 at least one strip per SM, else tiles                   */
+                                 order 7, a few time steps, checkpoints every few steps;
+                                 5 takes the resident kernels there too), and, for the
+                                 rest, strips when the batch has at least one strip per
+                                 SM, else tiles                                          */
   int32_t strip_bands;        /* strip kernel: element rows per CTA; 0 = automatic
                                  (full-height strips when the batch's strips give 2
                                  CTAs per SM, else chunks of >= 4 rows so that strips

@@ -799,11 +799,12 @@ bool ticks_win(const sem_solve_t* sv, const std::vector<int>& cls, int sms) {
   const sem_plan_s* p0 = sv[cls[0]].plan;
   const bool adj = sv[cls[0]].flags & SEM_F_ADJOINT, stc = p0->bnd_n > 0;
   long long elements = 0, chunks = 0, points = 0;
-  int nt = 0;
+  int nt = 0, k = 0;  // longest solve, longest segment of one that is replayed in several
   for (int i : cls) {
     const sem_plan_s* p = sv[i].plan;
     points += p->npoints;
     nt = std::max(nt, p->nt);
+    k = std::max(k, adj && sv[i].ckpt_k > 0 && sv[i].ckpt_k < p->nt ? (int)sv[i].ckpt_k : INT_MAX);
     elements += (long long)p->nelx * p->nelz;
     chunks += (long long)strips_of(p, nullptr) * ((p->nelz + kMinChunk - 1) / kMinChunk);
   }
@@ -813,6 +814,12 @@ bool ticks_win(const sem_solve_t* sv, const std::vector<int>& cls, int sms) {
   // 0.25 -> 0.28 (12 steps 0.41 -> 0.35); 128 of them, 12 steps 1.19 -> 1.41 (24 steps 2.0, both); gradients
   // 0.14 -> 0.18 (0.19, both), 0.67 -> 0.80 (1.10 -> 1.02), 3.2 -> 3.6 (5.3 -> 5.0).
   if (nt <= 5.0 + 1.2e-6 * (double)points) return true;
+  // So has each segment's replay and adjoint, which a short explicit interval repeats every k steps: 300
+  // steps, k = 2, 40x20: order 2 4.8 -> 4.9 ms, order 3 4.9 -> 6.5 (k = 3: 4.9 -> 4.7), order 4 5.1 -> 5.7 (5.1
+  // -> 4.4), order 5 5.8 -> 10.6 (k = 3: 5.8 -> 8.0; k = 4 and 4 models: 6.8, both); 30x15, order 6, k = 6
+  // 5.7 -> 7.1 (k = 10: 5.7 -> 5.9, 4 models 7.5 -> 5.9), order 7, k = 10 6.2 -> 9.4 (k = 16, 4 models: 8.3 -> 8.7).
+  static const int shortest[8] = {0, 2, 2, 3, 3, 4, 8, 16};
+  if (k < shortest[p0->npol]) return true;
   if (p0->npol == 7) {
     // A lane's element of order 7 does not fit its registers (500 to 1200 bytes spilled): 6 us a forward
     // step and 10 an adjoint one, however small the tile.  Where a tick takes its least time too it is

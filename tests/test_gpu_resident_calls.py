@@ -76,6 +76,15 @@ def test_memory_budget_is_for_automatic_intervals(mode, kw):
     (4, (100, 50), 8, 33, "sponge", "gradient", {}, "strip"),
     (4, (20, 10), 6, 1, "sponge", "forward", {}, "resident"),
     (4, (100, 50), 9, 33, "sponge", "gradient", {}, "resident"),
+    (4, (20, 10), 30, 1, "sponge", "gradient", {"ckpt_k": 2}, "tile"),      # short segments
+    (4, (20, 10), 30, 1, "sponge", "gradient", {"ckpt_k": 3}, "resident"),
+    (5, (20, 10), 30, 2, "stacey", "gradient", {"ckpt_k": 3}, "tile"),
+    (5, (20, 10), 30, 2, "stacey", "gradient", {"ckpt_k": 4}, "resident"),
+    (6, (20, 10), 30, 1, "sponge", "gradient", {"ckpt_k": 7}, "tile"),
+    (6, (20, 10), 30, 1, "sponge", "gradient", {"ckpt_k": 8}, "resident"),
+    (2, (20, 10), 30, 1, "sponge", "gradient", {"ckpt_k": 2}, "resident"),
+    (7, (57, 29), 30, 2, "sponge", "gradient", {"ckpt_k": 15}, "tile"),
+    (7, (57, 29), 30, 2, "sponge", "gradient", {"ckpt_k": 16}, "resident"),
     (7, (11, 6), 40, 1, "sponge", "gradient", {}, "resident"),
     (7, (23, 11), 40, 1, "sponge", "forward", {}, "resident"),
     (7, (57, 29), 40, 2, "stacey", "gradient", {}, "resident"),
