@@ -160,8 +160,10 @@ int sem_run(sem_batch_t* batch, const sem_solve_t* solves, int32_t n,
             const sem_launch_cfg_t* cfg, void* stream);
 /* number of kernel launches issued by the last sem_run (for accounting) */
 int64_t sem_batch_last_launches(const sem_batch_t* batch);
-/* number of consecutive groups the last sem_run ran: waves of the resident kernels and
- * groups of the others (1 unless ckpt_k = 0 solves were split under the memory budget) */
+/* number of consecutive groups the last sem_run ran: waves of the resident kernels (of
+ * several classes of solves by order, boundary mode and adjoint, one after another; as many
+ * as do not fit the SMs at once) and groups of the others (1 unless ckpt_k = 0 solves were
+ * split under the memory budget) */
 int32_t sem_batch_last_groups(const sem_batch_t* batch);
 /* launch shape the last sem_run used: tile of the tile or resident kernels (elements) and
  * strip kernel element rows per CTA (0 otherwise); any pointer may be NULL */
@@ -194,6 +196,10 @@ int sem_forward_adjoint(sem_batch_t* batch, const sem_plan_t* plan, const double
  * kernel's tick barrier); 2: a grid barrier that completes.  Blocks about 2 s for
  * 0 and 1; *status_out = SEM_ERR_TIMEOUT for 0 and 1, SEM_OK for 2. */
 int sem_selftest_wait(int32_t which, int32_t* status_out);
+/* The same for the resident kernels' exchange words: the batch's next wave of tiles that is
+ * not a cluster is launched without its last tile, whose neighbours' waits then run out
+ * (about 2 s); the solve reports SEM_ERR_TIMEOUT. */
+int sem_selftest_drop_tile(sem_batch_t* batch);
 /* Host only: the receivers, injected receivers, quads of nodes and terms of the fullest tile
  * of a resident tiling (tiles_x x tiles_z balanced tiles), as counted when the tiling is
  * chosen and as found in the lists that it runs with.  rec_base: (x, z) node of each

@@ -57,7 +57,7 @@ EXPORTS = ["sem_plan_create", "sem_plan_destroy", "sem_plan_workspace_bytes", "s
            "sem_batch_destroy", "sem_run", "sem_batch_last_launches", "sem_batch_last_kernel",
            "sem_batch_last_groups", "sem_batch_last_shape", "sem_batch_last_ticks",
            "sem_batch_last_tick_ms", "sem_forward",
-           "sem_forward_adjoint", "sem_forward_noalloc", "sem_selftest_wait", "sem_selftest_receivers",
+           "sem_forward_adjoint", "sem_forward_noalloc", "sem_selftest_wait", "sem_selftest_receivers", "sem_selftest_drop_tile",
            "sem_selftest_fail_marches", "sem_engine_create", "sem_engine_destroy",
            "sem_engine_submit", "sem_engine_step", "sem_engine_status", "sem_engine_release",
            "sem_engine_stats", "sem_velocity_from_curve", "sem_project_from_curve",
@@ -104,6 +104,7 @@ def load(path=None):
     lib.sem_forward_adjoint.argtypes = [vp, vp, vp, vp, dbl, i32, i32, vp, vp, vp, vp]
     lib.sem_forward_noalloc.argtypes = [vp, vp, vp, vp, vp]
     lib.sem_selftest_wait.argtypes = [i32, vp]
+    lib.sem_selftest_drop_tile.argtypes = [vp]
     lib.sem_selftest_receivers.argtypes = [i32, i32, i32, i32, vp, i32, i32, vp, vp]
     lib.sem_selftest_fail_marches.argtypes = [vp, i32, i32]
     lib.sem_engine_create.argtypes = [C.POINTER(EngineCfg), C.POINTER(vp)]

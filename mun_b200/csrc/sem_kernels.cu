@@ -2476,6 +2476,7 @@ struct sem_batch_s {
   unsigned ll_tag = 0;
   bool ll_recorded = false;             //   a captured run's launches may be replayed, with their tags
   int fail_skip = 0, fail_groups = 0;   // diagnostics: resident groups that run, then groups that fail
+  bool drop_tile = false;               //   and the next cooperative wave is launched without its last tile
   char* d_sync = nullptr;               // persistent strip kernel: per-CTA tick counters and
   long long sync_cap = 0;               //   per-solve barrier counters
 };
@@ -3281,6 +3282,12 @@ int sem_selftest_wait(int32_t which, int32_t* status_out) {
   cudaFree(buf);
   *status_out = h;
   return rc;
+}
+
+int sem_selftest_drop_tile(sem_batch_t* b) {
+  if (!b) return fail(SEM_ERR_ARG, "null argument");
+  b->drop_tile = true;
+  return SEM_OK;
 }
 
 int sem_selftest_receivers(int32_t npol, int32_t nelx, int32_t nelz, int32_t nrec, const int32_t* rec_base,

@@ -732,7 +732,9 @@ int run_res_group(sem_batch_t* b, const sem_solve_t* sv, char* const* at, const 
         b->ll_tag = 0;
       }
       cudaLaunchConfig_t lc = {};
-      lc.gridDim = dim3((unsigned)v.ncta);
+      const bool drop = b->drop_tile && !v.cluster && v.ncta > 1;
+      b->drop_tile = b->drop_tile && !drop;
+      lc.gridDim = dim3((unsigned)(v.ncta - drop));
       lc.blockDim = dim3((unsigned)(v.h.nc + v.h.nio));
       lc.dynamicSmemBytes = (size_t)v.L.total * 4;
       lc.stream = stream;

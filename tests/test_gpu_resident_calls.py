@@ -1,11 +1,13 @@
 """Calls that the resident kernels take over from the tick kernels: what callers could do with
 those, they can do with these."""
+import time
+
 import numpy as np
 import pytest
 import torch
 
-from mun_b200 import Batch, SEMPlan
-from tests.test_gpu_resident import _plan, _same, _spec
+from mun_b200 import Batch, SEMPlan, _lib
+from tests.test_gpu_resident import _compare, _plan, _same, _spec
 
 pytestmark = pytest.mark.gpu
 
@@ -100,3 +102,61 @@ def test_automatic_kernel_is_the_faster_one(npol, shape, nt, models, boundary, m
     for r, s in zip(ref, got):
         assert int(r.status.item()) == int(s.status.item()) == 0 and torch.equal(r.rec, s.rec)
         assert r.grad is None or torch.equal(r.grad, s.grad)
+
+
+@pytest.mark.parametrize("window", [(13, 88, 3), (0, 20, 1), (90, 97, 2)])
+def test_stacey_edges_with_a_misfit_window(window):
+    # (the waves of the first 20 steps do not meet: that window's gradient is 0)
+    p, c = _plan(11, 12, 4, 97, 8, "stacey")
+    for k in (0, 7):
+        ref, got = (_spec(p, c, 3, "gradient", ckpt_k=k, window=window) for _ in range(2))
+        Batch(kernel=1).run([ref])
+        b = Batch(kernel=5)
+        b.run([got])
+        torch.cuda.synchronize()
+        assert b.last_kernel == "resident" and int(ref.status.item()) == int(got.status.item()) == 0
+        assert torch.equal(ref.rec, got.rec) and torch.equal(ref.loglik, got.loglik) and torch.equal(ref.grad, got.grad)
+        assert window[1] == 20 or float(got.grad.abs().max()) > 0.0
+
+
+@pytest.mark.parametrize("nelx,nelz,boundary", [(330, 171, "sponge"), (345, 180, "stacey")])
+def test_fields_in_memory_over_several_segments(nelx, nelz, boundary):
+    # an automatic interval below the number of steps: the adjoint fields pass from segment to segment
+    p, c = _plan(nelx, nelz, 4, 120, 8, boundary, circle=True)
+    b = _compare(lambda: [_spec(p, c, 3, "gradient")], memory_budget=p.workspace_bytes(13, 35))
+    assert b.last_ticks > 2 * 120 + 2  # steps were replayed
+
+
+@pytest.mark.parametrize("kernel", [1, 2])
+def test_schedule_of_ticks_with_explicit_and_forward_solves(kernel):
+    # explicit intervals and forward solves keep their settings inside a batch that ticks run in groups
+    p, c = _plan(20, 10, 3, 90, 7, circle=True)
+
+    def make(k, k1):
+        return [_spec(p, c, i, "gradient", ckpt_k=(k, k1)[i == 1]) for i in range(4)] + [_spec(p, c, 9, "forward")]
+    ref, got, b = make(90, 90), make(0, 7), Batch(kernel=kernel)
+    Batch(kernel=5).run(ref)
+    b.run(got, memory_budget=int(0.6 * (3 * p.workspace_bytes(13, 13) + p.workspace_bytes(13, 7) + p.workspace_bytes(0, 2))))
+    torch.cuda.synchronize()
+    assert b.last_groups >= 2 and b.last_kernel == {1: "tile", 2: "strip"}[kernel]
+    _same(ref, got)
+
+
+def test_exchange_wait_gives_up_with_status():
+    # a tile that never runs: its neighbours' waits for its words run out, and the next call is right again
+    p, c = _plan(60, 30, 4, 40, 9, circle=True)
+    b, ref, got = Batch(kernel=5), _spec(p, c, 1, "forward"), _spec(p, c, 1, "forward")
+    Batch(kernel=1).run([ref])
+    b.run([got])
+    torch.cuda.synchronize()
+    assert b.last_kernel == "resident"
+    _same([ref], [got])
+    _lib.check(b._lib.sem_selftest_drop_tile(b.handle))
+    t0 = time.perf_counter()
+    b.run([got])
+    torch.cuda.synchronize()
+    dt = time.perf_counter() - t0
+    assert int(got.status.item()) == _lib.SEM_ERR_TIMEOUT and 1.5 < dt < 30.0
+    b.run([got])
+    torch.cuda.synchronize()
+    _same([ref], [got])
