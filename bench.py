@@ -49,6 +49,22 @@ BYTES_PER_NODE_ADJ_TICK = 36
 IMPL_BYTES_PER_NODE = {"forward_tick": 20, "adjoint_tick": 32.5}
 # and the resident kernels: the forward history written and read, a float64 fold every 16 steps
 RESIDENT_BYTES_PER_NODE = {"forward_step": 4, "adjoint_step": 5}
+
+
+def ops_per_node_step(N):
+    """fp32 operations of a forward and an adjoint step per node of order N: both directions' line
+    operators D^T (beta c^2 (D u)), 16 for the update, and the adjoint's sensitivities."""
+    NP = N + 1
+    step = 2 * (4 * NP * NP + 2 * NP) / N + 16
+    return 2 * step + 2 * (2 * NP * NP + 2 * NP) / N + 6
+
+
+def fp32_peak():
+    """TFLOP/s of the fp32 pipes, nominal: 128 fused multiply-adds per SM and clock."""
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count * 256 * peaks()[0].get("sm_max_mhz", 1965.0) / 1e6
+
+
 # DRAM bytes per node and tick of the strip kernel from one ncu capture (dram__bytes_read +
 # dram__bytes_write of one forward and one adjoint tick of a 128-model group, 10.3 M nodes),
 # scaled to a launch by its nodes
@@ -556,6 +572,7 @@ def run_single(args, steps=None, warmup=None, cpu_sample=None, emit=True):
                 ms.append(ev0.elapsed_time(ev1))
         return float(np.mean(ms)), s, b.last_ticks, b.last_tick_ms()
     m, s, ticks_k250, tick_ms = timed(250)
+    kernel_k250, shape_k250 = b.last_kernel, list(b.last_shape)
     # the same solve under the automatic schedule: its float32 forward history (25.6 GB)
     # fits, so there is no replay
     m_auto, s2, ticks_auto, tick_ms_auto = timed(0)
@@ -572,11 +589,17 @@ def run_single(args, steps=None, warmup=None, cpu_sample=None, emit=True):
     alg = BYTES_PER_NODE_STEP_FWDADJ * plan.npoints * nt
     pk, pk_kind = peaks()
     peak = float(pk.get("hbm_gbs", 6650.0))
+
+    def fractions(ms, kernel):
+        # the state of a resident march stays on chip (but for increment and gradient of this mesh's
+        # adjoint, which stay in L2): its fp32 operations; by ticks: the bytes of every tick
+        if kernel == "resident":
+            tf = ops_per_node_step(N) * plan.npoints * nt / (ms / 1e3) / 1e12
+            return {"achieved_tflops_fp32": tf, "fp32_frac": tf / fp32_peak()}
+        return {"achieved_gbs_56B": alg / (ms / 1e3) / 1e9, "hbm_frac_56B": alg / (ms / 1e3) / 1e9 / peak}
     auto = {"ms_per_solve": m_auto, "solves_per_s": 1e3 / m_auto, "ticks": ticks_auto,
-            "groups": b.last_groups, "bitwise_equal_to_k250": same,
-            "achieved_gbs_56B": alg / (m_auto / 1e3) / 1e9,
-            "hbm_frac_56B": alg / (m_auto / 1e3) / 1e9 / peak,
-            "tick_loop_ms": tick_ms_auto}
+            "kernel": b.last_kernel, "groups": b.last_groups, "bitwise_equal_to_k250": same,
+            **fractions(m_auto, b.last_kernel), "tick_loop_ms": tick_ms_auto}
     cpu = None
     if cpu_sample > 0:
         kw_o = dict(xmin=0.0, xmax=8000.0, zmin=0.0, zmax=4000.0, nelx=nelx, nelz=nelz, npol=N,
@@ -588,10 +611,9 @@ def run_single(args, steps=None, warmup=None, cpu_sample=None, emit=True):
                "sample": f"{cpu_sample}- and {2 * cpu_sample}-step runs of {nt}, linear fit "
                          f"(float64 state, no checkpointing: {el:.0f} s)"}
     out = {"workload": "single large solve: 400x200 el, N=4, 1,282,401 nodes, 5000 steps, k=250",
-           "nt": nt, "ms_per_solve": m, "solves_per_s": 1e3 / m, "kernel": b.last_kernel,
-           "shape (tile_ex, tile_ez, strip_bands)": list(b.last_shape),
-           "mnode_steps_per_s": plan.npoints * nt / (m / 1e3) / 1e6,
-           "achieved_gbs_56B": alg / (m / 1e3) / 1e9, "hbm_frac_56B": alg / (m / 1e3) / 1e9 / peak,
+           "nt": nt, "ms_per_solve": m, "solves_per_s": 1e3 / m, "kernel": kernel_k250,
+           "shape (tile_ex, tile_ez, strip_bands)": shape_k250,
+           "mnode_steps_per_s": plan.npoints * nt / (m / 1e3) / 1e6, **fractions(m, kernel_k250),
            "peak_kind": pk_kind, "ticks": ticks_k250, "tick_loop_ms": tick_ms,
            "auto_schedule": auto, "persistent_strip": pers, "cpu": cpu,
            "status": int(s.status.item()) | int(s2.status.item()) | int(s3.status.item())}
@@ -840,19 +862,46 @@ def main():
     # is the plain path's figure (the mean is reported beside it)
     plain_value = 1e3 / float(np.median(plain_ms))
 
-    # ---------------- roofline of the dominant kernel (the tick kernel, one launch per tick)
+    # ---------------- roofline of the dominant kernel
     pk, pk_kind = peaks()
-    alg_bytes = BYTES_PER_NODE_STEP_FWDADJ * W["npoints"] * W["nt"] * n
-    step_achieved = alg_bytes / (ms / 1e3) / 1e9
-    achieved = kern_bytes / (tick_loop_ms / 1e3) / 1e9
     peak = float(pk.get("hbm_gbs", 6650.0))
-    # DRAM traffic per node of each tick kind from the ncu capture of the strip kernel
-    # (128 models, per node), averaged over the step's ticks like the algorithmic bytes
-    traffic = None
-    if kernel_used == "strip" and TRAFFIC_B_PER_NODE:
-        traffic = W["npoints"] * (n // groups_used) * (
-            TRAFFIC_B_PER_NODE["fwd"] * fwd_like + TRAFFIC_B_PER_NODE["adj"] * groups_used * W["nt"]
-        ) / ticks_per_step
+    node_steps = W["npoints"] * W["nt"] * n
+    roofline = {"kernel": f"sem_{kernel_used}_kernel<4>", "traffic": None,
+                "launch_us_avg": 1e3 * tick_loop_ms / ticks_per_step,  # resident: a wave's step
+                "ticks_per_step": ticks_per_step, "forward_like_ticks": fwd_like}
+    if resident:
+        # one launch per wave of solves and sweep, state on chip: fp32 operations, and the forward
+        # history's bytes
+        top, ops = fp32_peak(), ops_per_node_step(4)
+        moved = sum(RESIDENT_BYTES_PER_NODE.values())
+        tf = [ops * node_steps / (t / 1e3) / 1e12 for t in (tick_loop_ms, ms)]
+        gbs = moved * node_steps / (tick_loop_ms / 1e3) / 1e9
+        roofline.update({
+            "bound": "fp32", "achieved": tf[0], "peak": top, "unit": "TFLOP/s", "frac": tf[0] / top,
+            "peak_kind": "nominal (SMs x 256 operations a clock x maximum clock)", "operations_per_node_step": ops,
+            "hbm": {"kernel_bytes_per_node_step": moved, "achieved": gbs, "unit": "GB/s", "frac": gbs / peak,
+                    "peak_kind": pk_kind},
+            "note": "fp32 operations of the step over the CUDA-event time of its marches",
+            "step_level": {"achieved": tf[1], "frac": tf[1] / top}})
+    else:
+        alg_bytes = BYTES_PER_NODE_STEP_FWDADJ * node_steps
+        step_achieved = alg_bytes / (ms / 1e3) / 1e9
+        achieved = kern_bytes / (tick_loop_ms / 1e3) / 1e9
+        # DRAM traffic per node of each tick kind from the ncu capture of the strip kernel
+        # (128 models, per node), averaged over the step's ticks like the algorithmic bytes
+        if kernel_used == "strip" and TRAFFIC_B_PER_NODE:
+            roofline["traffic"] = W["npoints"] * (n // groups_used) * (
+                TRAFFIC_B_PER_NODE["fwd"] * fwd_like + TRAFFIC_B_PER_NODE["adj"] * groups_used * W["nt"]
+            ) / ticks_per_step
+        roofline.update({
+            "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+            "peak_kind": pk_kind, "bytes_per_node_step": BYTES_PER_NODE_STEP_FWDADJ,
+            "bytes_per_node": {"forward_tick": BYTES_PER_NODE_FWD_TICK, "adjoint_tick": BYTES_PER_NODE_ADJ_TICK},
+            "kernel_bytes_per_node": IMPL_BYTES_PER_NODE,
+            "note": "algorithmic bytes (56 per fwd+adj node-step) of the step's tick launches over the "
+                    "CUDA-event time of the tick loops (one launch per tick; traffic = ncu DRAM bytes per launch)",
+            "step_level": {"bytes_per_node_step": BYTES_PER_NODE_STEP_FWDADJ, "achieved": step_achieved,
+                           "frac": step_achieved / peak}})
 
     # ---------------- parity of two of the models against the float64 oracle (host)
     parity = None
@@ -908,24 +957,7 @@ def main():
             "mnode_steps_per_s": W["npoints"] * W["nt"] * n * world / (ms / 1e3) / 1e6,
             "e2e": {"value": n * world / (e2e / 1e3), "unit": "solves/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h)},
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "traffic": traffic, "peak_kind": pk_kind,
-                         "kernel": f"sem_{kernel_used}_kernel<4>",
-                         "bytes_per_node_step": BYTES_PER_NODE_STEP_FWDADJ,
-                         "bytes_per_node": {"forward_tick": BYTES_PER_NODE_FWD_TICK,
-                                            "adjoint_tick": BYTES_PER_NODE_ADJ_TICK},
-                         "kernel_bytes_per_node": RESIDENT_BYTES_PER_NODE if resident else IMPL_BYTES_PER_NODE,
-                         # resident: a wave's step
-                         "launch_us_avg": 1e3 * tick_loop_ms / ticks_per_step,
-                         "ticks_per_step": ticks_per_step, "forward_like_ticks": fwd_like,
-                         "note": "algorithmic bytes (56 per fwd+adj node-step) of the step's tick "
-                                 "launches over the CUDA-event time of the tick loops (resident "
-                                 "kernels: one launch per wave of solves and sweep, state on chip; "
-                                 "tick kernels: one launch per tick, traffic = ncu DRAM bytes per "
-                                 "launch)",
-                         "step_level": {"bytes_per_node_step": BYTES_PER_NODE_STEP_FWDADJ,
-                                        "achieved": step_achieved,
-                                        "frac": step_achieved / peak}},
+            "roofline": roofline,
             "cpu_baseline": cpu,
             "parity": parity,
             **extras,
