@@ -6,7 +6,8 @@ batch: the same meshes, orders, receivers and velocities with a few dozen time s
 The checkpoint interval and group split stay with the library's memory-budget schedule.
 The choice is cached per batch signature (mesh sizes, orders, solve count, adjoint or
 not).  Results never depend on the choice: every variant computes bitwise the same
-numbers, so tuning only moves time.
+numbers, so tuning only moves time.  The resident kernels, which ``Batch()`` takes by itself
+for solves that fit the SMs, are not among the candidates.
 """
 from __future__ import annotations
 

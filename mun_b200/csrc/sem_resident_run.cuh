@@ -789,7 +789,8 @@ int sm_count(int device) {
   return sms;
 }
 // The class a solve runs resident in, or 0.  Adjoint solves too large for shared memory that were
-// given a checkpoint interval keep the strip kernel, whose schedule the interval was chosen for.
+// given a checkpoint interval keep the strip kernel, as they had it before (a replay with fields in
+// memory was not timed).
 int res_class(const sem_solve_t& s, int sms) {
   const int need = res_need(s.plan, s.flags & SEM_F_ADJOINT, sms);
   return need == RES_MEM && s.ckpt_k > 0 && s.ckpt_k < s.plan->nt ? 0 : need;

@@ -2,8 +2,8 @@
 
 A ``SolveSpec`` describes one solve: a plan, a nodal velocity on the device (float64,
 reference node order) and what to compute.  ``Batch.run`` executes any list of specs
-— mixed meshes, orders, step counts — as one tick-driven launch sequence, optionally
-replayed from captured CUDA graphs, and fills the specs' output tensors.
+— mixed meshes, orders, step counts — as resident marches or as one tick-driven launch
+sequence, optionally replayed from captured CUDA graphs, and fills the specs' output tensors.
 """
 import ctypes as C
 from dataclasses import dataclass, field
@@ -73,7 +73,8 @@ class Batch:
     def __init__(self, tile=(0, 0), threads=256, graph_chunk=0, kernel=0, strip_bands=0, autotune=False):
         """``autotune=True``: each ``run`` takes its kernel, tile shape or strip chunk height
         and graph chunk from ``mun_b200.autotune.tune`` for the batch's signature (timed once
-        per signature on a short proxy, then cached); results do not depend on the choice."""
+        per signature on a short proxy, then cached); results do not depend on the choice.
+        Its candidates are the tick kernels, not the resident ones that ``kernel=0`` takes."""
         lib = _lib.load()
         h = C.c_void_p()
         _lib.check(lib.sem_batch_create(C.byref(h)))
