@@ -805,6 +805,7 @@ bool ticks_win(const sem_solve_t* sv, const std::vector<int>& cls, int sms) {
   int nt = 0, k = 0;  // longest solve, longest segment of one that is replayed in several
   for (int i : cls) {
     const sem_plan_s* p = sv[i].plan;
+    if (p->nrec > std::min(kStripInj, kMaxInj)) return false;  // (strips and tiles may refuse more in one place)
     points += p->npoints;
     nt = std::max(nt, p->nt);
     k = std::max(k, adj && sv[i].ckpt_k > 0 && sv[i].ckpt_k < p->nt ? (int)sv[i].ckpt_k : INT_MAX);
@@ -851,10 +852,21 @@ int run_resident(sem_batch_t* b, const sem_solve_t* sv, char* const* at, int n, 
     if (!need) rest->push_back(i);
     else classes[std::make_tuple(p->npol, p->bnd_n > 0, adj, need)].push_back(i);
   }
+  long long by_ticks = 0;  // bytes of the workspaces that the tick kernels then hold at once
   for (auto& kv : classes) {
     if (!all && ticks_win(sv, kv.second, sms)) {
-      rest->insert(rest->end(), kv.second.begin(), kv.second.end());
-      continue;
+      long long bytes = 0;
+      int ns;
+      for (int i : kv.second) {
+        const bool adj = sv[i].flags & SEM_F_ADJOINT;
+        const int k = adj ? std::max(2, std::min((int)sv[i].ckpt_k, sv[i].plan->nt)) : 2;
+        if (!adj || sv[i].ckpt_k > 0) bytes += layout(sv[i].plan, sv[i].flags, k, &ns).bytes;
+      }
+      if (by_ticks + bytes <= budget) {  // (these split no batch without an automatic interval)
+        by_ticks += bytes;
+        rest->insert(rest->end(), kv.second.begin(), kv.second.end());
+        continue;
+      }
     }
     const std::vector<ResGroup> groups = res_plan(sv, kv.second, sms, budget);
     if (groups.empty()) { rest->insert(rest->end(), kv.second.begin(), kv.second.end()); continue; }

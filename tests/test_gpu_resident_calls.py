@@ -160,3 +160,21 @@ def test_exchange_wait_gives_up_with_status():
     b.run([got])
     torch.cuda.synchronize()
     _same([ref], [got])
+
+
+@pytest.mark.parametrize("npol,shape,nt,models,mode,kw", [
+    (4, (100, 50), 5, 16, "forward", {}), (5, (60, 30), 20, 24, "gradient", {"ckpt_k": 2})])
+def test_what_ticks_refuse_stays_resident(npol, shape, nt, models, mode, kw):
+    # more receivers in one strip's band than strips take, in batches that are faster by ticks
+    p, c = _plan(*shape, npol, nt, 1)
+    p = SEMPlan(**dict(p.kwargs, receivers=np.stack([np.linspace(3.0, 340.0, 300), np.full(300, 10.0)], 1)))
+    ref, got = ([_spec(p, c, 3 + i, mode, **kw) for i in range(models)] for _ in range(2))
+    with pytest.raises(ValueError):
+        Batch(kernel=2).run([_spec(p, c, 3, mode, **kw)])
+    Batch(kernel=5).run(ref)
+    b = Batch()
+    b.run(got)
+    torch.cuda.synchronize()
+    assert b.last_kernel == "resident"
+    for r, s in zip(ref, got):
+        assert torch.equal(r.rec, s.rec) and (r.grad is None or torch.equal(r.grad, s.grad))
