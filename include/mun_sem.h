@@ -37,7 +37,8 @@ enum {
   SEM_ERR_ARG = 1,        /* bad argument (reference: ValueError)                    */
   SEM_ERR_CUDA = 2,       /* CUDA runtime error                                      */
   SEM_ERR_OOM = 3,        /* device allocation failed                                */
-  SEM_ERR_NONFINITE = 4,  /* NaN/Inf detected in a wavefield (reported per solve)    */
+  SEM_ERR_NONFINITE = 4,  /* NaN/Inf detected in a wavefield (reported per solve; how
+                             far it spread into the gradient depends on the kernel)  */
   SEM_ERR_TIMEOUT = 5,    /* a bounded device wait gave up                           */
   SEM_ERR_UNSUPPORTED = 6 /* polynomial order outside 1..7                           */
 };
@@ -241,7 +242,8 @@ int sem_forward_noalloc(const sem_plan_t* plan, const double* velocity, float* r
  * of the resident kernels, while at most one earlier march is unfinished on the stream.
  * The others (too large, longer than that, or with a kernel or tile given) run side by
  * side by ticks, ticks_per_step with each call.  A solve's results do not depend on what
- * runs beside it (bitwise).  One thread uses an engine at a time.
+ * runs beside it (bitwise; by ticks, but for the rounding order at nodes between two element
+ * rows where receivers of both rows alternate).  One thread uses an engine at a time.
  * ------------------------------------------------------------------------------- */
 typedef struct sem_engine_s sem_engine_t;
 typedef struct {
