@@ -3606,7 +3606,13 @@ int engine_march(sem_engine_s* e, std::vector<EngineJob*>* admitted, cudaStream_
       done[of[i]] = 1;
     }
   }
-  CUDA_TRY(cudaEventRecord(end, stream));
+  if (std::find(done.begin(), done.end(), 1) == done.end()) {  // no march
+    e->marches.pop_back();
+    cudaEventDestroy(end);
+  } else {
+    const cudaError_t err = cudaEventRecord(end, stream);
+    if (err != cudaSuccess && !rc) rc = fail(SEM_ERR_CUDA, cudaGetErrorString(err));
+  }
   size_t keep = 0;
   for (size_t i = 0; i < admitted->size(); ++i) {
     EngineJob* j = (*admitted)[i];
